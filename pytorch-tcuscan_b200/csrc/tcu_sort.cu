@@ -1,10 +1,8 @@
-// tcu_sort.cu -- radix sort, top-k and the top-k pivot estimator on B200.
+// tcu_sort.cu -- radix sort and the top-k pivot estimator on B200.
 //
 // Reference: run_radix_sort (src/torch/torch_sort.h:30-82, kernels in
 // src/radix_sort.cpp:37-175) sorts 16-bit keys with sixteen one-bit stable
-// split passes; run_topk_int16 / run_topk_fp16 (src/torch/torch_topk.h:86-211,
-// src/kernels/kernel_topk.h:35-140) bisect the value range with repeated
-// splits; run_topk_pivot_fp16 (torch_topk.h:35-73,
+// split passes; run_topk_pivot_fp16 (torch_topk.h:35-73,
 // src/kernels/kernel_topk_pivot.h:22-160) estimates a lower bound of the k-th
 // largest value from sampled 32-element groups.
 //
@@ -17,14 +15,6 @@
 //                ballots, sorts the tile by digit in shared memory and writes
 //                each digit's run at the chunk's running position, so stores
 //                are runs of consecutive addresses.
-//   top-k        a radix select: 256-bin histograms of the key's high byte,
-//                then of the low byte inside the chosen high byte, fix the
-//                k-th largest key t; a count pass, one offset scan and an
-//                emit pass then write every element with key > t and the
-//                lowest-indexed elements with key == t, in index order.
-//                That is the set the reference's bisection returns (its
-//                splits are stable, so the ties it keeps are the first ones
-//                in input order); the reference emits it band by band.
 //   pivot        one CTA per block of tiles, one warp per 32-element group.
 // Keys are order-preserving unsigned images of the input bits: signed
 // integers flip the sign bit, floats flip all bits of negatives and set the
@@ -366,227 +356,6 @@ __global__ void __launch_bounds__(kRsThreads, 3) rs_scatter_kernel(const K* __re
 }
 
 // ---------------------------------------------------------------------------
-// Top-k over 16-bit keys.  The selection key merges -0 with +0 and maps every
-// NaN to the largest key: the reference compares values (x <= pivot is false
-// for NaN, so NaNs always rank above the pivot).
-enum TopkCodec { kTopkInt16 = 1, kTopkFp16 = 2, kTopkBf16 = 3 };
-
-template <int CODEC>
-__device__ __forceinline__ uint32_t topk_key(uint16_t b) {
-  if constexpr (CODEC == kTopkInt16) {
-    return (uint32_t)(b ^ 0x8000u);
-  } else {
-    const uint32_t em = CODEC == kTopkFp16 ? 0x7C00u : 0x7F80u;  // exponent field
-    if ((b & em) == em && (b & ~em & 0x7FFFu)) return 0xFFFFu;  // NaN
-    if ((b & 0x7FFFu) == 0) return 0x8000u;                     // +-0
-    return (b & 0x8000u) ? (uint32_t)(uint16_t)~b : (uint32_t)(b | 0x8000u);
-  }
-}
-
-struct TopkState {
-  int hi;            // high byte of the k-th largest key
-  int krem;          // elements still to take inside that high byte
-  int thr;           // the k-th largest key
-  int ties;          // elements equal to thr to take (lowest positions first)
-  long long above;   // elements above thr
-  int pad[10];
-};
-static_assert(sizeof(TopkState) == 64, "state");
-
-// 16 consecutive elements from e0 (16-byte vector loads when VEC and the
-// run is inside the array; elements past the end read as 0).
-template <bool VEC>
-__device__ __forceinline__ void load16(const uint16_t* __restrict__ x, int64_t e0, int64_t n, uint16_t (&v)[16]) {
-  if (VEC && e0 + 16 <= n) {
-    const uint4 a = __ldg(reinterpret_cast<const uint4*>(x + e0));
-    const uint4 b = __ldg(reinterpret_cast<const uint4*>(x + e0) + 1);
-    const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      v[2 * i] = (uint16_t)(w[i] & 0xFFFFu);
-      v[2 * i + 1] = (uint16_t)(w[i] >> 16);
-    }
-  } else {
-#pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = e0 + i < n ? x[e0 + i] : (uint16_t)0;
-  }
-}
-
-template <int CODEC, int LEVEL>
-struct TopkDigit {
-  int hi;
-  __device__ __forceinline__ int operator()(uint16_t b) const {
-    const uint32_t k = topk_key<CODEC>(b);
-    if (LEVEL == 0) return (int)(k >> 8);
-    return (int)(k >> 8) == hi ? (int)(k & 0xFF) : -1;
-  }
-};
-
-// 256-bin histogram of the key's high byte (LEVEL 0), or of the low byte
-// among keys whose high byte is st->hi (LEVEL 1), over contiguous chunks of
-// tiles; bins must be zero on entry.
-template <int CODEC, int LEVEL, bool VEC>
-__global__ void __launch_bounds__(kRsThreads) topk_hist_kernel(const uint16_t* __restrict__ x, int64_t n,
-                                                               int64_t num_tiles, const TopkState* __restrict__ st,
-                                                               unsigned* __restrict__ bins) {
-  __shared__ int s_h[kHistCopies * kRsDigits];
-#pragma unroll
-  for (int k = 0; k < kHistCopies; ++k) s_h[k * kRsDigits + threadIdx.x] = 0;
-  __syncthreads();
-  const int64_t tpc = chunk_tiles(num_tiles, gridDim.x);
-  const int64_t e_lo = blockIdx.x * tpc * kRsTile;
-  int64_t e_hi = e_lo + tpc * kRsTile;
-  e_hi = e_hi < n ? e_hi : n;
-  smem_hist_range<uint16_t, VEC>(x, e_lo, e_hi, s_h, TopkDigit<CODEC, LEVEL>{LEVEL ? st->hi : 0});
-  __syncthreads();
-  const int c = smem_hist_total(s_h);
-  if (c) atomicAdd(&bins[threadIdx.x], (unsigned)c);
-}
-
-// One CTA: the bin holding the k-th largest key, from the top of the histogram.
-template <int LEVEL>
-__global__ void __launch_bounds__(kRsThreads) topk_pick_kernel(const unsigned* __restrict__ bins, long long k,
-                                                               TopkState* st) {
-  __shared__ int sw[kRsWarps];
-  __shared__ int s_suffix[kRsDigits + 1];
-  const int d = threadIdx.x;
-  // suffix sums: s_suffix[d] = keys in bins >= d (scan of the reversed bins)
-  const int c = (int)bins[kRsDigits - 1 - d];
-  int tot;
-  const int pre = block_excl_scan256(c, sw, &tot);
-  s_suffix[kRsDigits - 1 - d] = pre + c;
-  if (d == 0) s_suffix[kRsDigits] = 0;
-  __syncthreads();
-  const long long want = LEVEL == 0 ? k : (long long)st->krem;
-  if ((long long)s_suffix[d] >= want && (long long)s_suffix[d + 1] < want) {
-    const int above = s_suffix[d + 1];
-    if (LEVEL == 0) {
-      st->hi = d;
-      st->krem = (int)(want - above);
-      st->above = above;
-    } else {
-      st->thr = (st->hi << 8) | d;
-      st->ties = (int)(want - above);
-      st->above += above;
-    }
-  }
-}
-
-// Per tile: elements above thr and equal to thr -- one warp per tile (each
-// lane 128 consecutive elements in 16-byte loads, all in flight), a warp sum,
-// no block barrier.
-template <int CODEC, bool VEC>
-__global__ void __launch_bounds__(kRsThreads) topk_count_kernel(const uint16_t* __restrict__ x, int64_t n,
-                                                                int64_t num_tiles, const TopkState* __restrict__ st,
-                                                                int* __restrict__ c_above, int* __restrict__ c_tie) {
-  const int lane = threadIdx.x & 31;
-  const uint32_t thr = (uint32_t)st->thr;
-  const int64_t warps = (int64_t)gridDim.x * kRsWarps;
-  for (int64_t t = (int64_t)blockIdx.x * kRsWarps + (threadIdx.x >> 5); t < num_tiles; t += warps) {  // warp-uniform
-    int aq = 0;  // above in the low half, equal in the high half
-#pragma unroll
-    for (int q = 0; q < kRsTile / 32 / 16; ++q) {  // 8 runs of 16 elements per lane
-      const int64_t e0 = t * kRsTile + ((int64_t)q * 32 + lane) * 16;
-      uint16_t v[16];
-      load16<VEC>(x, e0, n, v);
-#pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        const uint32_t k = topk_key<CODEC>(v[j]);
-        const bool in = e0 + j < n;
-        aq += (in && k > thr) ? 1 : ((in && k == thr) ? 0x10000 : 0);
-      }
-    }
-    aq = warp_sum_any(aq);
-    if (lane == 0) {
-      c_above[t] = aq & 0xFFFF;
-      c_tie[t] = aq >> 16;
-    }
-  }
-}
-
-// One CTA: per tile, the ties before it and the output offset (taken =
-// above + the ties still wanted); off[num_tiles] = k.
-__global__ void __launch_bounds__(kRsThreads) topk_offsets_kernel(const int* __restrict__ c_above,
-                                                                  const int* __restrict__ c_tie, int64_t num_tiles,
-                                                                  const TopkState* __restrict__ st,
-                                                                  int* __restrict__ tie_before, int* __restrict__ off) {
-  __shared__ int sw[kRsWarps];
-  const int ties = st->ties;
-  const int64_t per = (num_tiles + kRsThreads - 1) / kRsThreads;
-  const int64_t b0 = (int64_t)threadIdx.x * per;
-  const int64_t b1 = b0 + per < num_tiles ? b0 + per : num_tiles;
-  int qs = 0;
-  for (int64_t t = b0; t < b1; ++t) qs += c_tie[t];
-  int tot;
-  int q = block_excl_scan256(qs, sw, &tot);
-  int ss = 0;
-  for (int64_t t = b0; t < b1; ++t) {
-    const int c = c_tie[t];
-    int take = ties - q;
-    take = take < 0 ? 0 : (take > c ? c : take);
-    ss += c_above[t] + take;
-    q += c;
-  }
-  int s = block_excl_scan256(ss, sw, &tot);
-  q -= qs;  // back to this thread's first tile
-  for (int64_t t = b0; t < b1; ++t) {
-    const int c = c_tie[t];
-    int take = ties - q;
-    take = take < 0 ? 0 : (take > c ? c : take);
-    tie_before[t] = q;
-    off[t] = s;
-    s += c_above[t] + take;
-    q += c;
-  }
-  if (threadIdx.x == kRsThreads - 1) off[num_tiles] = s;
-}
-
-// Emits the selected elements of every tile in index order (values and int32
-// positions).  Tiles with nothing selected are skipped without reading them.
-template <int CODEC, bool VEC>
-__global__ void __launch_bounds__(kRsThreads) topk_emit_kernel(const uint16_t* __restrict__ x, int64_t n,
-                                                               int64_t num_tiles, const TopkState* __restrict__ st,
-                                                               const int* __restrict__ tie_before,
-                                                               const int* __restrict__ off, int64_t k,
-                                                               uint16_t* __restrict__ out, int* __restrict__ idx_out) {
-  __shared__ int sw[kRsWarps];
-  const uint32_t thr = (uint32_t)st->thr;
-  const int ties = st->ties;
-  for (int64_t t = blockIdx.x; t < num_tiles; t += gridDim.x) {
-    const int o0 = off[t];
-    if (off[t + 1] == o0) continue;  // block-uniform
-    const int64_t e0 = t * kRsTile + (int64_t)threadIdx.x * kRsEpt;  // 16 consecutive elements per thread
-    uint16_t xv[16];
-    load16<VEC>(x, e0, n, xv);
-    unsigned am = 0, qm = 0;
-#pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      const uint32_t kk = topk_key<CODEC>(xv[j]);
-      const bool in = e0 + j < n;
-      am |= (unsigned)(in && kk > thr) << j;
-      qm |= (unsigned)(in && kk == thr) << j;
-    }
-    int tot;
-    // ties of this thread that are still wanted: the first (ties - rank) of them
-    const int tr = tie_before[t] + block_excl_scan256(__popc(qm), sw, &tot);
-    int want = ties - tr;
-    want = want < 0 ? 0 : want;
-    unsigned take = qm;
-    for (int c = __popc(qm); c > want; --c) take &= ~(1u << (31 - __clz(take)));  // drop the last ties
-    const unsigned selm = am | take;
-    int o = o0 + block_excl_scan256(__popc(selm), sw, &tot);
-#pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      if (((selm >> j) & 1u) && o < k) {
-        out[o] = xv[j];
-        idx_out[o] = (int)(e0 + j);
-        ++o;
-      }
-    }
-  }
-}
-
-// ---------------------------------------------------------------------------
 // Top-k pivot estimator (kernel_topk_pivot.h:96-160).  Block b reads up to
 // 8 tiles of num_samples * 32 elements from tile b * tiles_per_block on; per
 // tile, each 32-element group gives its k_inner-th largest value, those
@@ -721,55 +490,6 @@ static tcu_status_t radix_sort_t(const K* x, int64_t n, K* out, int* idx_out, ui
   return TCU_OK;
 }
 
-static int rs_grid(int64_t tiles, int per_sm) {
-  int64_t g = (int64_t)sm_count() * per_sm;
-  if (tiles < g) g = tiles;
-  return (int)(g < 1 ? 1 : g);
-}
-
-// tmp layout: bins[2][256] | state | c_above[T] | c_tie[T] | tie_before[T] | off[T + 1]
-static size_t topk_tmp_bytes(int64_t n) {
-  const int64_t T = rs_tiles(n);
-  return 2048 + sizeof(TopkState) + 3 * align256((size_t)T * 4) + align256((size_t)(T + 1) * 4);
-}
-
-template <int CODEC>
-static tcu_status_t topk_t(const uint16_t* x, int64_t n, int64_t k, uint16_t* out, int* idx_out, uint8_t* tmp,
-                           cudaStream_t st) {
-  const bool VEC = aligned16(x);
-  const int64_t T = rs_tiles(n);
-  unsigned* bins = reinterpret_cast<unsigned*>(tmp);
-  TopkState* state = reinterpret_cast<TopkState*>(tmp + 2048);
-  int* c_above = reinterpret_cast<int*>(tmp + 2048 + sizeof(TopkState));
-  int* c_tie = reinterpret_cast<int*>(reinterpret_cast<uint8_t*>(c_above) + align256((size_t)T * 4));
-  int* tie_before = reinterpret_cast<int*>(reinterpret_cast<uint8_t*>(c_tie) + align256((size_t)T * 4));
-  int* off = reinterpret_cast<int*>(reinterpret_cast<uint8_t*>(tie_before) + align256((size_t)T * 4));
-  cudaError_t e = cudaMemsetAsync(tmp, 0, 2048 + sizeof(TopkState), st);
-  if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync(topk state)");
-  const int g = rs_grid(T, 8);
-  const int gw = rs_grid((T + kRsWarps - 1) / kRsWarps, 8);  // a warp per tile
-  const int gh = rs_grid(T, 6);  // histogram CTAs: contiguous chunks of tiles, 32 KB of counters
-  if (VEC) {
-    topk_hist_kernel<CODEC, 0, true><<<gh, kRsThreads, 0, st>>>(x, n, T, state, bins);
-    topk_pick_kernel<0><<<1, kRsThreads, 0, st>>>(bins, k, state);
-    topk_hist_kernel<CODEC, 1, true><<<gh, kRsThreads, 0, st>>>(x, n, T, state, bins + 256);
-    topk_pick_kernel<1><<<1, kRsThreads, 0, st>>>(bins + 256, k, state);
-    topk_count_kernel<CODEC, true><<<gw, kRsThreads, 0, st>>>(x, n, T, state, c_above, c_tie);
-    topk_offsets_kernel<<<1, kRsThreads, 0, st>>>(c_above, c_tie, T, state, tie_before, off);
-    topk_emit_kernel<CODEC, true><<<g, kRsThreads, 0, st>>>(x, n, T, state, tie_before, off, k, out, idx_out);
-  } else {
-    topk_hist_kernel<CODEC, 0, false><<<gh, kRsThreads, 0, st>>>(x, n, T, state, bins);
-    topk_pick_kernel<0><<<1, kRsThreads, 0, st>>>(bins, k, state);
-    topk_hist_kernel<CODEC, 1, false><<<gh, kRsThreads, 0, st>>>(x, n, T, state, bins + 256);
-    topk_pick_kernel<1><<<1, kRsThreads, 0, st>>>(bins + 256, k, state);
-    topk_count_kernel<CODEC, false><<<gw, kRsThreads, 0, st>>>(x, n, T, state, c_above, c_tie);
-    topk_offsets_kernel<<<1, kRsThreads, 0, st>>>(c_above, c_tie, T, state, tie_before, off);
-    topk_emit_kernel<CODEC, false><<<g, kRsThreads, 0, st>>>(x, n, T, state, tie_before, off, k, out, idx_out);
-  }
-  e = cudaGetLastError();
-  return e == cudaSuccess ? TCU_OK : cuda_fail(e, "topk launch");
-}
-
 static int pivot_blocks(int64_t n, int num_samples, int64_t* tiles_per_block, int64_t* num_tiles) {
   const int64_t tile_len = (int64_t)num_samples * 32;
   const int64_t T = (n + tile_len - 1) / tile_len;
@@ -820,27 +540,6 @@ tcu_status_t tcu_radix_sort(const void* x, tcu_dtype_t dtype, int64_t n, void* o
     case TCU_INT32: return radix_sort_t<uint32_t, kCodecSigned>((const uint32_t*)x, n, (uint32_t*)out, idx_out, t, st);
     default: return radix_sort_t<uint32_t, kCodecFloat>((const uint32_t*)x, n, (uint32_t*)out, idx_out, t, st);
   }
-}
-
-size_t tcu_topk_tmp_bytes(int64_t n) { return n <= 0 ? 0 : topk_tmp_bytes(n); }
-
-tcu_status_t tcu_topk(const void* x, tcu_dtype_t dtype, int64_t n, int64_t k, void* out, int32_t* idx_out, void* tmp,
-                      size_t tmp_bytes, void* stream) {
-  if (n < 0 || n > 0x7FFFFFFFLL || k < 0 || k > n) return TCU_ERR_ARG;
-  if (dtype != TCU_INT16 && dtype != TCU_FLOAT16 && dtype != TCU_BFLOAT16) return TCU_ERR_DTYPE;
-  if (k == 0) return TCU_OK;
-  if (!x || !out || !idx_out) return TCU_ERR_ARG;
-  if (!tmp || tmp_bytes < topk_tmp_bytes(n)) return TCU_ERR_WORKSPACE;
-  if ((reinterpret_cast<uintptr_t>(tmp) & 255u) || (reinterpret_cast<uintptr_t>(idx_out) & 3u) ||
-      (reinterpret_cast<uintptr_t>(x) & 1u) || (reinterpret_cast<uintptr_t>(out) & 1u))
-    return TCU_ERR_ALIGN;
-  cudaStream_t st = (cudaStream_t)stream;
-  const uint16_t* xs = static_cast<const uint16_t*>(x);
-  uint16_t* o = static_cast<uint16_t*>(out);
-  uint8_t* t = static_cast<uint8_t*>(tmp);
-  if (dtype == TCU_INT16) return topk_t<kTopkInt16>(xs, n, k, o, idx_out, t, st);
-  if (dtype == TCU_FLOAT16) return topk_t<kTopkFp16>(xs, n, k, o, idx_out, t, st);
-  return topk_t<kTopkBf16>(xs, n, k, o, idx_out, t, st);
 }
 
 int tcu_topk_pivot_blocks(int64_t n, int num_samples) {
