@@ -292,6 +292,20 @@ TCU_API tcu_status_t tcu_compress_count(const int8_t* mask, int64_t n, int elem_
 TCU_API tcu_status_t tcu_compress_counted(const void* x, int elem_bytes, const int8_t* mask, int64_t n,
                                           const void* idx_in, int idx_bytes, int idx_mode, void* out, void* idx_out,
                                           int64_t capacity, void* ws, size_t ws_bytes, void* stream);
+/* The two halves again, for callers with scratch of their own: `tmp` of
+ * tcu_compact_tmp_bytes(n) bytes (16-byte aligned; n / 8 bytes and a little)
+ * takes the mask as one bit per element beside the counts, so that the
+ * compaction reads n / 8 bytes of bits instead of n bytes of mask, and no
+ * look-back workspace is touched.  tcu_compact_count writes the total (int64)
+ * to count_dev when given; tcu_compact_counted takes the same n, tmp and
+ * stream.  split != 0: the stable partition of tcu_split (idx_mode 0 or 1,
+ * outputs of n elements, capacity not read).                              */
+TCU_API size_t tcu_compact_tmp_bytes(int64_t n);
+TCU_API tcu_status_t tcu_compact_count(const int8_t* mask, int64_t n, void* count_dev, void* tmp, size_t tmp_bytes,
+                                       void* stream);
+TCU_API tcu_status_t tcu_compact_counted(const void* x, int elem_bytes, int64_t n, const void* idx_in, int idx_bytes,
+                                         int idx_mode, int split, void* out, void* idx_out, int64_t capacity,
+                                         void* tmp, size_t tmp_bytes, void* stream);
 /* Compaction of several independent requests packed into one buffer (the
  * serving loop batches compress calls this way): the stable compaction of
  * x[mask != 0] over all n elements, plus seg_pos[i] = number of selected

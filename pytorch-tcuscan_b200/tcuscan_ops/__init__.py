@@ -219,15 +219,12 @@ def _compress(x, mask, out_len, idx_in=None, idx_mode=0, idx_dtype=torch.int32, 
     elif idx_mode == 2:
         ib = torch.empty((), dtype=idx_dtype).element_size()
     sp = stream_ptr(x.device)
-    from tcuscan_b200 import autotune
-
-    autotune.apply_ctas(autotune.best("compress", x.dtype, n)[1])
-    ws, wsb = workspace(x.device, _lib.lib.tcu_workspace_bytes(n, 64))
-    counted = out_len is None
-    if counted:
-        cnt = torch.empty(1, dtype=torch.int64, device=x.device)
-        check(_lib.lib.tcu_compress_count(mask.data_ptr(), n, x.element_size(), idx_mode, ib, cnt.data_ptr(), ws, wsb,
-                                          sp), where)
+    tb = _lib.lib.tcu_compact_tmp_bytes(n)
+    tmp = torch.empty(tb, dtype=torch.uint8, device=x.device)
+    cnt = torch.empty(1, dtype=torch.int64, device=x.device) if out_len is None else None
+    check(_lib.lib.tcu_compact_count(mask.data_ptr(), n, cnt.data_ptr() if cnt is not None else None, tmp.data_ptr(),
+                                     tb, sp), where)
+    if cnt is not None:
         out_len = int(cnt.item())
     z = torch.empty(out_len, dtype=x.dtype, device=x.device)
     idx_out = None
@@ -240,12 +237,8 @@ def _compress(x, mask, out_len, idx_in=None, idx_mode=0, idx_dtype=torch.int32, 
     zp = z.data_ptr() if out_len > 0 else x.data_ptr()
     ip = (idx_out.data_ptr() if out_len > 0 else x.data_ptr()) if idx_out is not None else None
     inp = idx_in.data_ptr() if idx_in is not None else None
-    if counted:
-        st = _lib.lib.tcu_compress_counted(x.data_ptr(), x.element_size(), mask.data_ptr(), n, inp, ib, idx_mode, zp,
-                                           ip, out_len, ws, wsb, sp)
-    else:
-        st = _lib.lib.tcu_compress(x.data_ptr(), x.element_size(), mask.data_ptr(), n, inp, ib, idx_mode, zp, ip,
-                                   out_len, None, ws, wsb, sp)
+    st = _lib.lib.tcu_compact_counted(x.data_ptr(), x.element_size(), n, inp, ib, idx_mode, 0, zp, ip, out_len,
+                                      tmp.data_ptr(), tb, sp)
     check(st, where)
     _after(x)
     return z, idx_out
@@ -327,16 +320,16 @@ def _split(x, mask, indices_in, where):
     idx_out = torch.empty_like(indices_in) if indices_in is not None else None
     if n == 0:
         return z, idx_out
-    from tcuscan_b200 import autotune
-
-    autotune.apply_ctas(autotune.best("compress", x.dtype, n)[1])
     ib = indices_in.element_size() if indices_in is not None else 0
-    ws, wsb = workspace(x.device, _lib.lib.tcu_workspace_bytes(n, 64))
-    check(_lib.lib.tcu_split(x.data_ptr(), x.element_size(), mask.data_ptr(), n,
-                             indices_in.data_ptr() if indices_in is not None else None, ib,
-                             1 if indices_in is not None else 0, z.data_ptr(),
-                             idx_out.data_ptr() if idx_out is not None else None, None, ws, wsb,
-                             stream_ptr(x.device)), where)
+    sp = stream_ptr(x.device)
+    tb = _lib.lib.tcu_compact_tmp_bytes(n)
+    tmp = torch.empty(tb, dtype=torch.uint8, device=x.device)
+    check(_lib.lib.tcu_compact_count(mask.data_ptr(), n, None, tmp.data_ptr(), tb, sp), where)
+    check(_lib.lib.tcu_compact_counted(x.data_ptr(), x.element_size(), n,
+                                       indices_in.data_ptr() if indices_in is not None else None, ib,
+                                       1 if indices_in is not None else 0, 1, z.data_ptr(),
+                                       idx_out.data_ptr() if idx_out is not None else None, n, tmp.data_ptr(), tb,
+                                       sp), where)
     _after(x)
     return z, idx_out
 
