@@ -10,8 +10,9 @@
 //   bm_tile_first_kernel  one warp per tile: the first bound at or after the
 //                         tile start (a 32-way search);
 //   bm_segsum_kernel      one CTA per tile, 64 bytes of input per thread
-//                         (32 elements for fp32 and for SpMV: it gathers x[cols] and
-//                         multiplies in FP32), loads issued first.  The
+//                         (32 elements for fp32 and for SpMV, whose products
+//                         x[cols] * vals are formed in FP32 with coalesced
+//                         loads and left in shared memory), loads issued first.  The
 //                         tile's bounds set two bitmaps in shared memory, one
 //                         bit per element: segment starts and segment ends
 //                         (the last element of every non-empty segment).
@@ -126,7 +127,7 @@ __device__ __forceinline__ int64_t bm_lower_bound(const IT* bounds, int64_t lo, 
 // int32 for int8); CT: cross-tile carry type; SPMV: element i is
 // vals[i] * x[cols[i]] (FP32 product), else vals[i].
 template <typename VT, typename ACC, typename CT, bool SPMV, typename IT>
-__global__ void __launch_bounds__(kBmThreads, SPMV ? 3 : (sizeof(VT) == 4 ? 4 : 6)) bm_segsum_kernel(const VT* __restrict__ vals,
+__global__ void __launch_bounds__(kBmThreads, SPMV ? 5 : (sizeof(VT) == 4 ? 4 : 6)) bm_segsum_kernel(const VT* __restrict__ vals,
                                                                   const int32_t* __restrict__ cols,
                                                                   const VT* __restrict__ x, int64_t x_len,
                                                                   const IT* __restrict__ bounds, int64_t nb,
@@ -146,51 +147,68 @@ __global__ void __launch_bounds__(kBmThreads, SPMV ? 3 : (sizeof(VT) == 4 ? 4 : 
   const int64_t c = blockIdx.x;
   const int64_t t0 = c * TILE;
   const int64_t t1 = t0 + TILE < n ? t0 + TILE : n;
-  const int64_t j0 = t0 + (int64_t)t * IPT;
-  const int nvalid = j0 >= t1 ? 0 : (j0 + IPT <= t1 ? IPT : (int)(t1 - j0));
 
-  // ---- the thread's elements: loads issued before the bounds work ----
+  // ---- the tile's elements: loads issued before the bounds work ----
   constexpr int WORDS = SPMV ? 1 : IPT * (int)sizeof(VT) / 4;
   uint32_t raw[WORDS];
-  int32_t cc[SPMV ? IPT : 1];
-  float pv[SPMV ? IPT : 1];
-  const bool vec = nvalid == IPT && ((reinterpret_cast<uintptr_t>(vals) & 15u) == 0) &&
-                   (!SPMV || (reinterpret_cast<uintptr_t>(cols) & 15u) == 0);
   if constexpr (SPMV) {
-    if (vec) {
+    // Products in FP32, kBmThreads * 4 elements at a time with coalesced loads,
+    // into the rows of the threads that sum them.  Bound by the rate of the x
+    // gathers; a thread loading its own 32 elements touched a line per lane in
+    // every load and held 80 registers, so three CTAs per SM took turns with
+    // them: 139 us for 17.2 M nonzeros (fp32, Zipf rows), 119 us with five
+    // CTAs of 48 registers (4 CTAs: 122 us; 6 CTAs spill: 190 us).
+    constexpr int BATCH = 4;
+    const bool vec = ((reinterpret_cast<uintptr_t>(vals) | reinterpret_cast<uintptr_t>(cols)) & 15u) == 0;
+#pragma unroll 1
+    for (int b = 0; b < TILE; b += kBmThreads * 4 * BATCH) {
+      int4 c4[BATCH];
+      float v4[BATCH][4];
 #pragma unroll
-      for (int q = 0; q < IPT / 4; ++q) {
-        const int4 c4 = __ldg(reinterpret_cast<const int4*>(cols + j0) + q);
-        cc[4 * q] = c4.x; cc[4 * q + 1] = c4.y; cc[4 * q + 2] = c4.z; cc[4 * q + 3] = c4.w;
-      }
-      if constexpr (sizeof(VT) == 4) {
-#pragma unroll
-        for (int q = 0; q < IPT / 4; ++q) {
-          const float4 v4 = __ldg(reinterpret_cast<const float4*>(vals + j0) + q);
-          pv[4 * q] = v4.x; pv[4 * q + 1] = v4.y; pv[4 * q + 2] = v4.z; pv[4 * q + 3] = v4.w;
-        }
-      } else {
-#pragma unroll
-        for (int q = 0; q < IPT / 8; ++q) {
-          const uint4 u = __ldg(reinterpret_cast<const uint4*>(vals + j0) + q);
-          const uint32_t uu[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-          for (int h = 0; h < 4; ++h) {
-            const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&uu[h]));
-            pv[8 * q + 2 * h] = f.x;
-            pv[8 * q + 2 * h + 1] = f.y;
+      for (int k = 0; k < BATCH; ++k) {
+        const int64_t e = t0 + b + (k * kBmThreads + t) * 4;
+        if (vec && e + 4 <= t1) {
+          c4[k] = __ldg(reinterpret_cast<const int4*>(cols + e));
+          if constexpr (sizeof(VT) == 4) {
+            const float4 f = __ldg(reinterpret_cast<const float4*>(vals + e));
+            v4[k][0] = f.x; v4[k][1] = f.y; v4[k][2] = f.z; v4[k][3] = f.w;
+          } else {
+            const uint2 u = __ldg(reinterpret_cast<const uint2*>(vals + e));
+            const float2 f0 = __half22float2(*reinterpret_cast<const __half2*>(&u.x));
+            const float2 f1 = __half22float2(*reinterpret_cast<const __half2*>(&u.y));
+            v4[k][0] = f0.x; v4[k][1] = f0.y; v4[k][2] = f1.x; v4[k][3] = f1.y;
           }
+        } else {
+          int cc[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const bool in = e + i < t1;
+            cc[i] = in ? __ldg(cols + e + i) : 0;
+            v4[k][i] = in ? elem_f32<VT>(vals + e + i) : 0.f;
+          }
+          c4[k] = make_int4(cc[0], cc[1], cc[2], cc[3]);
         }
       }
-    } else {
 #pragma unroll
-      for (int i = 0; i < IPT; ++i) {
-        const bool in = i < nvalid;
-        cc[i] = in ? __ldg(cols + j0 + i) : 0;
-        pv[i] = in ? elem_f32<VT>(vals + j0 + i) : 0.f;
+      for (int k = 0; k < BATCH; ++k) {
+        const int e = b + (k * kBmThreads + t) * 4;
+        const int cc[4] = {c4[k].x, c4[k].y, c4[k].z, c4[k].w};
+        float pr[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          float xv = 0.f;
+          if ((unsigned long long)(unsigned)cc[i] < (unsigned long long)x_len) xv = elem_f32<VT>(x + cc[i]);
+          else if (t0 + e + i < t1 && ws) record_error(ws, TCU_ERR_ARG, 301, (uint32_t)(t0 + e + i));
+          pr[i] = __fmul_rn(v4[k][i], xv);
+        }
+        const int row = e >> 5, ch = (e >> 2) & 7;
+        *reinterpret_cast<float4*>(sP + row * 32 + 4 * (ch ^ (row & 7))) = make_float4(pr[0], pr[1], pr[2], pr[3]);
       }
     }
   } else {
+    const int64_t j0 = t0 + (int64_t)t * IPT;
+    const int nvalid = j0 >= t1 ? 0 : (j0 + IPT <= t1 ? IPT : (int)(t1 - j0));
+    const bool vec = nvalid == IPT && ((reinterpret_cast<uintptr_t>(vals) & 15u) == 0);
     if (vec) {
 #pragma unroll
       for (int q = 0; q < WORDS / 4; ++q) {
@@ -214,18 +232,6 @@ __global__ void __launch_bounds__(kBmThreads, SPMV ? 3 : (sizeof(VT) == 4 ? 4 : 
     }
   }
 
-  // ---- SpMV: gather x[cols] (FP32 products), issued before the bounds
-  // work so their L2 latency overlaps the chain first bound index ->
-  // bounds -> bitmaps ----
-  if constexpr (SPMV) {
-#pragma unroll
-    for (int i = 0; i < IPT; ++i) {
-      float xv = 0.f;
-      if ((unsigned long long)(unsigned)cc[i] < (unsigned long long)x_len) xv = elem_f32<VT>(x + cc[i]);
-      else if (i < nvalid && ws) record_error(ws, TCU_ERR_ARG, 301, (uint32_t)(j0 + i));
-      pv[i] = __fmul_rn(pv[i], xv);
-    }
-  }
   // ---- boundary bitmaps from the tile's bounds ----
 #pragma unroll
   for (int q = 0; q < WPT; ++q) {
@@ -282,9 +288,7 @@ __global__ void __launch_bounds__(kBmThreads, SPMV ? 3 : (sizeof(VT) == 4 ? 4 : 
   int ord = wpre + ecs - ec;
 
   auto elem = [&](int i) -> ACC {
-    if constexpr (SPMV) {
-      return pv[i];
-    } else if constexpr (sizeof(VT) == 1) {
+    if constexpr (sizeof(VT) == 1) {
       return (ACC)(int8_t)(raw[i >> 2] >> (8 * (i & 3)));
     } else if constexpr (sizeof(VT) == 2) {
       return (ACC)__half2float(__ushort_as_half((unsigned short)(raw[i >> 1] >> (16 * (i & 1)))));
@@ -321,10 +325,18 @@ __global__ void __launch_bounds__(kBmThreads, SPMV ? 3 : (sizeof(VT) == 4 ? 4 : 
     ACC pfx = ACC(0);
 #pragma unroll
     for (int i4 = 0; i4 < 8; ++i4) {
-      const ACC a0 = pfx + elem(q * 32 + 4 * i4);
-      const ACC a1 = a0 + elem(q * 32 + 4 * i4 + 1);
-      const ACC a2 = a1 + elem(q * 32 + 4 * i4 + 2);
-      const ACC a3 = a2 + elem(q * 32 + 4 * i4 + 3);
+      ACC el[4];
+      if constexpr (SPMV) {  // the products of the thread's row, replaced by their prefixes
+        const float4 f = *reinterpret_cast<const float4*>(myP + 4 * (i4 ^ sx));
+        el[0] = f.x; el[1] = f.y; el[2] = f.z; el[3] = f.w;
+      } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) el[i] = elem(q * 32 + 4 * i4 + i);
+      }
+      const ACC a0 = pfx + el[0];
+      const ACC a1 = a0 + el[1];
+      const ACC a2 = a1 + el[2];
+      const ACC a3 = a2 + el[3];
       if (need) {
         if constexpr (sizeof(ACC) == 4) {
           uint4 u;
