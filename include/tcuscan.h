@@ -422,6 +422,10 @@ typedef struct tcu_pack_item {
 } tcu_pack_item_t;
 TCU_API tcu_status_t tcu_pack(const tcu_pack_item_t* items, int64_t nitems, int src_bytes, int dst_bytes, void* dst,
                               int64_t total, void* stream);
+/* cudaMemcpyAsync between any two of device and pinned host memory on
+ * `stream`: the loop's copies of request tables and result positions, queued
+ * like its launches.  No reference counterpart.                            */
+TCU_API tcu_status_t tcu_copy_async(void* dst, const void* src, size_t bytes, void* stream);
 
 #ifdef __cplusplus
 }

@@ -175,4 +175,13 @@ tcu_status_t tcu_pack(const tcu_pack_item_t* items, int64_t nitems, int src_byte
   return TCU_ERR_DTYPE;
 }
 
+// One asynchronous copy between any two of device and pinned host memory, for
+// callers that queue their launches through this interface alone.
+tcu_status_t tcu_copy_async(void* dst, const void* src, size_t bytes, void* stream) {
+  if (bytes == 0) return TCU_OK;
+  if (!dst || !src) return TCU_ERR_ARG;
+  cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDefault, (cudaStream_t)stream);
+  return e == cudaSuccess ? TCU_OK : cuda_fail(e, "tcu_copy_async");
+}
+
 }  // extern "C"

@@ -36,6 +36,7 @@ results bit for bit, floating results within the scan family's tolerance
 their rows; only the order in which FP64 carries are added may differ).
 """
 import collections
+import contextlib
 import ctypes
 import time
 
@@ -64,6 +65,9 @@ BATCH_SLACK = 8192  # bytes per batch for buffer alignment inside its block
 
 # matches tcu_pack_item_t (include/tcuscan.h)
 PACK_ITEM = np.dtype([("src", "<u8"), ("dst", "<i8"), ("n", "<i8"), ("len", "<i8"), ("add", "<i8")])
+
+
+_HERE = contextlib.nullcontext()
 
 
 def _roundup(a, m):
@@ -113,7 +117,7 @@ class _Slot:
 
 
 class _Batch:
-    __slots__ = ("id", "cls", "ids", "slot", "off", "bytes", "out_off", "out_dtype", "out_len")
+    __slots__ = ("id", "cls", "ids", "slot", "off", "bytes", "out_off", "out_dtype", "out_len", "out")
 
 
 class Server:
@@ -177,6 +181,11 @@ class Server:
         self._next_arrival = 0  # requests [0, _next_arrival) have been moved to the class queues
         self.queues = collections.defaultdict(collections.deque)  # class -> deque of id arrays
         self._keepalive = {}
+
+    def __del__(self):
+        # the slots' streams may still read the pinned tables and the arena
+        for si in list(getattr(self, "inflight", ())):
+            self.slots[si].event.synchronize()
 
     # ---------------------------------------------------------------- table
     def _alloc(self, cap):
@@ -282,6 +291,18 @@ class Server:
         b = b + np.where(op == COMPRESS, npad * (1 + eb) + 8, 0)
         return b
 
+    def _class_bytes(self, ids):
+        """_bytes of requests of one class (op and dtype of the first)."""
+        npad = _roundup(self.n[ids], ALIGN)
+        i = ids[0]
+        eb, op = int(_EB[self.dt[i]]), int(self.op[i])
+        fixed = 2 * PACK_ITEM.itemsize + 16
+        if op == SCAN:
+            return npad * (eb + 4) + fixed
+        if op == SEG_SUM:
+            return npad * eb + (self.nseg[ids] + 1) * 12 + fixed
+        return npad * (1 + 2 * eb) + (fixed + 8)
+
     # ---------------------------------------------------------------- loop
     def _arrivals(self):
         t = self.now()
@@ -308,7 +329,7 @@ class Server:
         room -= BATCH_SLACK
         while q and count < self.max_batch:
             ids = q[0]
-            b = self._bytes(ids)
+            b = self._class_bytes(ids)  # a queue holds one class
             cum = np.cumsum(b)
             k = int(np.searchsorted(cum, room - used, side="right"))
             k = min(k, self.max_batch - count)
@@ -461,15 +482,14 @@ class Server:
         m_off = carve(mb)
         x_off = carve(total * eb)
         base = self.arena.base
-        ab = self.arena.buf
         st = sl.stream
         sp = ctypes.c_void_p(st.cuda_stream)
         S = tcuscan_ops._pick_S(self.S, dtype, max(total, 1), op="seg")
         L = _lib.lib
         wsp = sl.ws.data_ptr()
-        with torch.cuda.stream(st):
+        with (_HERE if torch.cuda.current_device() == self.dev.index else torch.cuda.device(self.dev)):
             if k:
-                ab[m_off:m_off + mb].copy_(sl.pinned[:mb], non_blocking=True)
+                tcuscan_ops.check(L.tcu_copy_async(base + m_off, sl.pinned.data_ptr(), mb, sp), "serve request table")
                 tcuscan_ops.check(L.tcu_pack(base + m_off, k, eb, eb, base + x_off, total, sp), "serve pack")
             if op == SCAN:
                 out_dtype = tcuscan_ops._scan_out_dtype(dtype)
@@ -530,14 +550,15 @@ class Server:
                 s_ = L.tcu_compress_segments(base + x_off, eb, base + mk_off, total, starts, k, base + z_off, total,
                                              base + p_off, wsp, sl.wsb, sp)
                 tcuscan_ops.check(s_, "serve compress")
-                sl.pos_host[: k + 1].copy_(ab[p_off:p_off + (k + 1) * 8].view(torch.int64), non_blocking=True)
+                tcuscan_ops.check(L.tcu_copy_async(sl.pos_host.data_ptr(), base + p_off, (k + 1) * 8, sp),
+                                  "serve compress positions")
                 out_len = total
             sl.event.record(st)
         if cur[0] - off > nbytes:
             raise AssertionError("batch layout overran its block")
         b = _Batch()
         b.id, b.cls, b.ids, b.slot, b.off, b.bytes = self.batches, cls, ids, si, off, nbytes
-        b.out_off, b.out_dtype, b.out_len = z_off, out_dtype, out_len
+        b.out_off, b.out_dtype, b.out_len, b.out = z_off, out_dtype, out_len, None
         self.bid[ids] = self.batches
         self.batches += 1
         self.inflight[si] = b
@@ -553,9 +574,10 @@ class Server:
         b = self.finished.get(int(self.bid[rid]))
         if b is None:
             raise KeyError(f"request {rid}: result released (keep_results=False or release() called)")
-        es = torch.empty((), dtype=b.out_dtype).element_size()
-        out = self.arena.buf[b.out_off:b.out_off + b.out_len * es].view(b.out_dtype)
-        return out[int(self.roff[rid]): int(self.roff[rid] + self.rlen[rid])]
+        if b.out is None:  # the batch's outputs as one typed view, once for all of its requests
+            b.out = self.arena.buf[b.out_off:b.out_off + b.out_len * b.out_dtype.itemsize].view(b.out_dtype)
+        off = int(self.roff[rid])
+        return b.out[off:off + int(self.rlen[rid])]
 
     def release(self):
         """Drop every kept batch and return its block to the arena."""

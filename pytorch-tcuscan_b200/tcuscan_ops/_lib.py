@@ -102,6 +102,7 @@ _sig("tcu_topk_tmp_bytes", _SZ, _I64)
 _sig("tcu_topk", _ST, _P, _I, _I64, _I64, _P, _P, _P, _SZ, _P)
 _sig("tcu_topk_pivot_blocks", _I, _I64, _I)
 _sig("tcu_topk_pivot", _ST, _P, _I, _I64, _I, _I, _I, _P, _P)
+_sig("tcu_copy_async", _ST, _P, _P, _SZ, _P)
 _sig("tcu_pack", _ST, _P, _I64, _I, _I, _P, _I64, _P)
 _sig("tcu_csr_gather", _ST, _P, _I, _P, _I64, _P, _I64, _P, _P, _P)
 _sig("tcu_gather_spmv", _ST, _P, _I, _I64, _P, _I, _I64, _P, _P, _P)
