@@ -10,6 +10,8 @@ device by ``tune()``:
                                                            fp16: 16..128), CTAs
     seg       batched uneven rows (sorted segment starts)  S (32/64), CTAs
     compress  tcuscan_ops.run_compress_pos                 CTAs
+              (the compaction takes a CTA per eight tiles whatever the cap, so its
+              entries record times only)
 
 Entries are keyed by op, dtype and floor(log2(n)); lookups use the nearest
 tuned size of the same op and dtype.  The table is JSON (``TCU_AUTOTUNE_CACHE``
