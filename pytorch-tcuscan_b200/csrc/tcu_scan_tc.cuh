@@ -1382,7 +1382,7 @@ __device__ __forceinline__ void seg_epilogue(const ScanParams& p, const CUtensor
       // as soon as the tile's data landed)
       if (MODE != kSegBounds && MODE != kSegPeriodic && wg_thread == 0)
         publish_aggregate<V>((int64_t)tid, run, runf, V(0), p.descs, epoch);
-      const V pre = wg_lookback<V>((int64_t)tid, run, V(0), p.descs, epoch, wc, &ctl->lb[g], wg_thread, bar_id,
+      const V pre = wg_lookback_nearest<V>((int64_t)tid, run, V(0), p.descs, epoch, wc, &ctl->lb[g], wg_thread, bar_id,
                                    runf);
 #pragma unroll
       for (int j = 0; j < BPT; ++j)
