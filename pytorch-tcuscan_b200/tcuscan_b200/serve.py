@@ -149,6 +149,15 @@ class Server:
         # per-slot look-back workspace sized for the largest batch, then the arena
         ws_need = int(max(_lib.lib.tcu_workspace_bytes(self.max_batch_bytes, 64),
                           _lib.lib.tcu_rows_workspace_bytes(self.max_batch_bytes)))
+        ws_total = ws_need * slots
+        if self.budget - ws_total < (1 << 20):
+            raise ValueError("serving budget too small for its workspaces")
+        # Workspaces and arena come from the allocator of the caller's current
+        # stream, so they may be memory that work queued there still uses (a
+        # temporary just freed): they are zeroed on that stream, and no slot
+        # starts before it gets here.  Zeroing them on the slots' own streams
+        # ran among a freed temporary's last kernels.
+        cur = torch.cuda.current_stream(self.dev)
         self.slots = []
         for i in range(slots):
             sl = _Slot()
@@ -159,13 +168,12 @@ class Server:
             sl.pos_host = torch.empty(max_batch + 1, dtype=torch.int64, pin_memory=True)
             sl.ws = torch.empty(ws_need, dtype=torch.uint8, device=self.dev)  # owned by the slot
             sl.wsb = ctypes.c_size_t(ws_need)
-            st_ = _lib.lib.tcu_workspace_init(sl.ws.data_ptr(), sl.wsb, ctypes.c_void_p(sl.stream.cuda_stream))
+            st_ = _lib.lib.tcu_workspace_init(sl.ws.data_ptr(), sl.wsb, ctypes.c_void_p(cur.cuda_stream))
             tcuscan_ops.check(st_, "serve workspace")
             self.slots.append(sl)
-        ws_total = ws_need * slots
-        if self.budget - ws_total < (1 << 20):
-            raise ValueError("serving budget too small for its workspaces")
         self.arena = Arena(self.budget - ws_total, self.dev)
+        for sl in self.slots:
+            sl.stream.wait_stream(cur)
         self.free_slots = collections.deque(range(slots))
         self.inflight = {}  # slot index -> _Batch
         self.finished = {}  # batch id -> _Batch (keep_results)

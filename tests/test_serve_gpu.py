@@ -259,3 +259,63 @@ def test_server_budget_admission_and_arrivals():
     s2.submit("scan", big)
     with pytest.raises(MemoryError):
         s2.run()
+
+
+def test_server_memory_follows_the_callers_stream():
+    """A server's workspaces may be memory of temporaries whose kernels are still queued on the caller's stream:
+    building and dropping servers behind such a chain changes nothing that the chain writes, and the workspaces
+    are as good as fresh ones."""
+    import tcuscan_ops
+    from tcuscan_b200 import serve
+
+    n = 17 << 20  # 68 MiB of int32: the four 16 MiB workspaces of a server fit the freed temporary
+    want = torch.arange(n, dtype=torch.int32, device=DEV) + 100
+    x = torch.randint(-8, 9, (300_000,), dtype=torch.int8, device=DEV)
+    ref = torch.cumsum(x.long(), 0).int()
+    torch.cuda.synchronize()
+    for _ in range(5):
+        dst = torch.zeros(n, dtype=torch.int32, device=DEV)
+        t = torch.arange(n, dtype=torch.int32, device=DEV)
+        for _ in range(100):  # a few milliseconds of queued work
+            t += 1
+        dst.copy_(t)
+        del t
+        for _ in range(3):
+            srv = serve.Server(DEV, budget_bytes=1 << 30, slots=4, max_batch_bytes=2 << 30, keep_results=True)
+            del srv
+        srv = serve.Server(DEV, budget_bytes=1 << 30, slots=4, max_batch_bytes=2 << 30, keep_results=True)
+        ids = [srv.submit("scan", x) for _ in range(8)]
+        srv.run()
+        assert torch.equal(dst, want)
+        assert all(torch.equal(srv.result(i), ref) for i in ids)
+    tcuscan_ops.raise_device_error(DEV)
+
+
+@pytest.mark.parametrize("seed", range(6))
+def test_burst_of_large_requests(seed):
+    """48 requests of up to 2^24 elements, all waiting at once, on a server built right behind the kernels that
+    fill the requests' pools: large scans and sums run in place, the rest packed, on four streams.  Integers and
+    compactions exact, floating results within 1e-3 of the 64-bit ones as everywhere in this file."""
+    from tcuscan_b200 import serve, workloads
+
+    st = workloads.ServedStream(48, DEV, 11 + seed, lo=1 << 10, hi=1 << 24)
+    for i, pool in enumerate(st.pools):
+        pool.copy_(workloads.scan_input(pool.numel(), pool.dtype, DEV, 1000 * seed + i))
+    srv = serve.Server(DEV, budget_bytes=8 << 30, keep_results=True)
+    ids = srv.submit_many(*st.arrays(), np.full(st.count, srv.now()))
+    srv.run()
+    for i, rid in enumerate(ids):
+        op, x, aux = st.request(i)
+        got = srv.result(rid)
+        if op == serve.COMPRESS:
+            assert torch.equal(got, x[aux.bool()]), i
+            continue
+        wide = torch.cumsum(x.long() if x.dtype == torch.int8 else x.double(), 0)
+        if op == serve.SEG_SUM:
+            wide = torch.cat([torch.zeros_like(wide[:1]), wide])[aux.long()]
+            wide = wide[1:] - wide[:-1]
+        if x.dtype == torch.int8:
+            assert torch.equal(got, wide.int()), i
+        else:
+            err = (got.double() - wide).abs() / wide.abs().clamp_min(1.0)
+            assert got.shape == wide.shape and float(err.max()) <= TOL, (i, op, x.dtype, x.numel())

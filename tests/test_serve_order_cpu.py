@@ -1,0 +1,155 @@
+"""Stream order of the serving loop, without a GPU.
+
+The server runs on a model of CUDA streams: every operation it queues (through
+the C interface or through torch) is written down with the set of operations
+that are certain to come before it -- those of its own stream and those that a
+recorded event or a stream wait brings along.  What the loop's correctness
+needs is then a statement about these sets: the operations a caller queued
+before must be in the set of every operation that reads or overwrites the same
+memory.
+"""
+import contextlib
+import types
+
+import numpy as np
+import pytest
+import torch
+
+
+class Stream:
+    made = 0
+
+    def __init__(self, model, name):
+        self.model, self.name, self.before = model, name, frozenset()
+        Stream.made += 1
+        self.cuda_stream = 1000 + Stream.made
+        model.streams[self.cuda_stream] = self
+
+    def op(self, what):
+        """Queue an operation; returns its id."""
+        i = len(self.model.ops)
+        self.model.ops.append((what, self, self.before))
+        self.before = self.before | {i}
+        return i
+
+    def wait_stream(self, other):
+        self.before = self.before | other.before
+
+    def wait_event(self, ev):
+        self.before = self.before | ev.point
+
+    def synchronize(self):
+        self.model.done |= self.before
+
+
+class Event:
+    def __init__(self, model):
+        self.model, self.point = model, frozenset()
+
+    def record(self, stream=None):
+        self.point = (stream or self.model.current).before
+
+    def query(self):
+        self.model.done |= self.point
+        return True
+
+    def synchronize(self):
+        self.model.done |= self.point
+
+
+class Model:
+    """Streams, and a C interface whose calls only queue operations."""
+
+    def __init__(self):
+        self.ops, self.streams, self.done, self.fail = [], {}, frozenset(), None
+        self.current = Stream(self, "caller")
+
+    def __getattr__(self, name):  # lib.tcu_*
+        if not name.startswith("tcu_"):
+            raise AttributeError(name)
+
+        def call(*args):
+            if name.endswith("_bytes"):
+                return 1 << 12
+            if name == self.fail:
+                return 3  # TCU_ERR_LAUNCH
+            self.streams[args[-1].value].op(name)
+            return 0
+
+        return call
+
+    def find(self, name):
+        return [(i, s, before) for i, (what, s, before) in enumerate(self.ops) if what == name]
+
+
+@pytest.fixture
+def model(monkeypatch):
+    from tcuscan_b200 import serve
+    from tcuscan_ops import _lib
+
+    m = Model()
+    cuda = types.SimpleNamespace(
+        current_device=lambda: 0, device=lambda d: contextlib.nullcontext(),
+        Stream=lambda dev=None: Stream(m, "slot"), Event=lambda enable_timing=False: Event(m),
+        current_stream=lambda dev=None: m.current, is_current_stream_capturing=lambda: False)
+
+    class Torch:
+        def __getattr__(self, name):
+            return getattr(torch, name)
+
+        @staticmethod
+        def empty(*a, **k):
+            k.pop("device", None)
+            k.pop("pin_memory", None)
+            return torch.zeros(*a, **k)
+
+    shim = Torch()
+    shim.cuda = cuda
+
+    class Lib:
+        def __getattr__(self, name):
+            return getattr(_lib, name)
+
+    lib = Lib()
+    lib.lib = m
+    monkeypatch.setattr(serve, "torch", shim)
+    monkeypatch.setattr(serve, "_lib", lib)
+    return m
+
+
+def _server(m, **kw):
+    from tcuscan_b200 import serve
+
+    return serve.Server("cuda:0", budget_bytes=4 << 20, slots=2, keep_results=True, **kw)
+
+
+def _submit(srv, op, n=5000, k=1):
+    """k int8 requests on memory of nobody's (the model reads nothing)."""
+    nseg = 40 if op == 1 else 0
+    return srv.submit_many(np.full(k, op, np.int8), np.zeros(k, np.int8), np.full(k, n), np.full(k, 4096, np.uint64),
+                           np.full(k, 8192, np.uint64), np.full(k, nseg), np.full(k, 4 if op == 1 else 0, np.int8),
+                           np.full(k, srv.now()))
+
+
+def test_construction_follows_the_callers_work(model):
+    """The workspaces and the arena may be memory that the caller's queued work still uses (a temporary just
+    freed): nothing of the server touches them before that work, and what the caller queues next on memory of a
+    server that is gone comes after the server's own."""
+    late = model.current.op("a temporary's last kernel")
+    srv = _server(model)
+    inits = model.find("tcu_workspace_init")
+    assert len(inits) == 2
+    for i, s, before in inits:
+        assert late in before
+        assert i in model.current.before  # the caller's next kernel may get this block again
+    for sl in srv.slots:
+        assert late in sl.stream.before and all(i in sl.stream.before for i, _, _ in inits)
+
+
+def test_a_refused_server_leaves_nothing_queued(model):
+    from tcuscan_b200 import serve
+
+    with pytest.raises(ValueError):
+        serve.Server("cuda:0", budget_bytes=1 << 16, slots=2)
+    for i, s, before in model.find("tcu_workspace_init"):
+        assert i in model.current.before
