@@ -27,6 +27,10 @@ its stream.  This module keeps the device busy with many requests at once:
   ``tcu_compress_segments`` (compress -- every compress request is packed,
   with its output offset).  Batches on different slots run on different
   CUDA streams and overlap on the GPU.
+- A batch follows, on the device, whatever the caller had queued on its
+  current stream when it submitted, released results or drove the loop: the
+  kernels that fill a request's inputs, and those that read results whose
+  blocks are used again.
 - Completion is read from one CUDA event per slot (polled, never a device
   synchronisation).  A request's result is a view of its batch's block.
 
@@ -113,7 +117,7 @@ class Arena:
 
 
 class _Slot:
-    __slots__ = ("idx", "stream", "event", "pinned", "pos_host", "ws", "wsb")
+    __slots__ = ("idx", "stream", "event", "pinned", "pos_host", "ws", "wsb", "seen")
 
 
 class _Batch:
@@ -132,6 +136,8 @@ class Server:
     timing        record completions on the device clock (``done_gpu``)
                   against the event of ``mark_start()``.
     """
+
+    _callers = None  # stream handle -> [event, call, stream] of the streams this server is called from
 
     def __init__(self, device="cuda", budget_bytes=24 << 30, slots=4, max_batch=4096, max_batch_bytes=None,
                  S=None, keep_results=False, timing=False):
@@ -168,12 +174,14 @@ class Server:
             sl.pos_host = torch.empty(max_batch + 1, dtype=torch.int64, pin_memory=True)
             sl.ws = torch.empty(ws_need, dtype=torch.uint8, device=self.dev)  # owned by the slot
             sl.wsb = ctypes.c_size_t(ws_need)
+            sl.seen = 0
             st_ = _lib.lib.tcu_workspace_init(sl.ws.data_ptr(), sl.wsb, ctypes.c_void_p(cur.cuda_stream))
             tcuscan_ops.check(st_, "serve workspace")
             self.slots.append(sl)
         self.arena = Arena(self.budget - ws_total, self.dev)
         for sl in self.slots:
             sl.stream.wait_stream(cur)
+        self._callers, self._calls = {}, 0
         self.free_slots = collections.deque(range(slots))
         self.inflight = {}  # slot index -> _Batch
         self.finished = {}  # batch id -> _Batch (keep_results)
@@ -237,6 +245,19 @@ class Server:
         self.start_event.record(torch.cuda.current_stream(self.dev))
         self.t0 = time.perf_counter()
 
+    def _after_caller(self):
+        """Batches launched from now on come after the work queued so far on
+        the caller's current stream."""
+        if self._callers is None or torch.cuda.is_current_stream_capturing():
+            return
+        h = _lib._stream_key(self.dev)[1]
+        c = self._callers.get(h)
+        if c is None:
+            c = self._callers[h] = [torch.cuda.Event(), 0, torch.cuda.current_stream(self.dev)]
+        c[0].record(c[2])
+        self._calls += 1
+        c[1] = self._calls
+
     def submit(self, op, x, aux=None, arrival=None):
         """Queue one request; returns its id.  op: "scan" | "seg_sum" | "compress".
         seg_sum takes a CSR row-pointer tensor (int32/int64, R + 1 entries,
@@ -272,7 +293,8 @@ class Server:
         uint64).  Arrival times (seconds since the server's clock started)
         must be non-decreasing; a request enters its queue once
         ``now() >= arrival``.  The caller keeps the data alive until the
-        requests complete."""
+        requests complete; data still being written on its current stream is
+        waited for on the device."""
         k = len(n)
         arrival = np.asarray(arrival, dtype=np.float64)
         if k and self._n and arrival[0] < self.arrival[self._n - 1]:
@@ -284,6 +306,7 @@ class Server:
         self.arrival[s] = arrival
         ids = np.arange(self._n, self._n + k, dtype=np.int64)
         self._n += k
+        self._after_caller()
         return ids
 
     # --------------------------------------------------------------- sizing
@@ -403,6 +426,8 @@ class Server:
             ids, nbytes = self._take(cls, room)
             if ids is None:
                 break  # the oldest class does not fit yet: wait for memory
+            if launched == 0:
+                self._after_caller()
             self._launch(cls, ids, nbytes)
             launched += 1
         return launched
@@ -495,6 +520,10 @@ class Server:
         S = tcuscan_ops._pick_S(self.S, dtype, max(total, 1), op="seg")
         L = _lib.lib
         wsp = sl.ws.data_ptr()
+        for ev, call, _ in self._callers.values():
+            if call > sl.seen:
+                st.wait_event(ev)
+        sl.seen = self._calls
         with (_HERE if torch.cuda.current_device() == self.dev.index else torch.cuda.device(self.dev)):
             if k:
                 tcuscan_ops.check(L.tcu_copy_async(base + m_off, sl.pinned.data_ptr(), mb, sp), "serve request table")
@@ -589,6 +618,7 @@ class Server:
 
     def release(self):
         """Drop every kept batch and return its block to the arena."""
+        self._after_caller()  # readers of the results precede the blocks' next use
         for b in self.finished.values():
             self._free(b)
         self.finished.clear()

@@ -319,3 +319,42 @@ def test_burst_of_large_requests(seed):
         else:
             err = (got.double() - wide).abs() / wide.abs().clamp_min(1.0)
             assert got.shape == wide.shape and float(err.max()) <= TOL, (i, op, x.dtype, x.numel())
+
+
+def test_requests_still_being_written_when_they_are_served():
+    """Inputs whose kernels are queued on the caller's stream (the current one, and a side stream at submit) and
+    results read by queued kernels when their blocks are released."""
+    from tcuscan_b200 import serve
+
+    n = 6_000_000  # above SOLO_MIN: in place; the others are packed
+    srv = serve.Server(DEV, budget_bytes=2 << 30, slots=4, keep_results=True)
+    side = torch.cuda.Stream(DEV)
+    base = torch.randint(-3, 4, (n,), dtype=torch.int8, device=DEV)
+    mask = (torch.rand(n, device=DEV) < 0.3).to(torch.int8)
+    for k in range(4):
+        x = torch.zeros(n, dtype=torch.int8, device=DEV)
+        big = torch.zeros(64 << 20, dtype=torch.int32, device=DEV)
+        torch.cuda.synchronize()
+        want = base + k
+        with torch.cuda.stream(side):
+            for _ in range(20):
+                big += 1
+            y = want[: 1 << 20] + 1
+            r3 = srv.submit("scan", y)
+        for _ in range(20):  # a few milliseconds in front of the input's own kernel
+            big.add_(1)
+        x.copy_(want)
+        r1 = srv.submit("scan", x)
+        r2 = srv.submit("compress", x[:1 << 20], mask[:1 << 20])
+        srv.run()
+        for _ in range(20):
+            big.add_(1)
+        got = [srv.result(r).clone() for r in (r1, r2, r3)]  # queued behind the adds
+        srv.release()
+        z = [srv.submit("scan", base) for _ in range(3)]  # its blocks are the released ones
+        srv.run()
+        assert torch.equal(got[0], torch.cumsum(want.long(), 0).int())
+        assert torch.equal(got[1], want[: 1 << 20][mask[: 1 << 20].bool()])
+        assert torch.equal(got[2], torch.cumsum(want[: 1 << 20].long() + 1, 0).int())
+        assert all(torch.equal(srv.result(i), torch.cumsum(base.long(), 0).int()) for i in z)
+        srv.release()

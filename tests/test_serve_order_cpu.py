@@ -112,6 +112,7 @@ def model(monkeypatch):
 
     lib = Lib()
     lib.lib = m
+    lib._stream_key = lambda dev: (0, m.current.cuda_stream)
     monkeypatch.setattr(serve, "torch", shim)
     monkeypatch.setattr(serve, "_lib", lib)
     return m
@@ -153,3 +154,44 @@ def test_a_refused_server_leaves_nothing_queued(model):
         serve.Server("cuda:0", budget_bytes=1 << 16, slots=2)
     for i, s, before in model.find("tcu_workspace_init"):
         assert i in model.current.before
+
+
+def test_batches_follow_the_work_that_fills_their_requests(model):
+    """Whatever a caller queued on its stream before submit(), before run() or -- on another stream -- before
+    submitting from there precedes every kernel of the batch."""
+    from tcuscan_b200 import serve
+
+    srv = _server(model)
+    early = model.current.op("input of the first request")
+    _submit(srv, serve.SCAN)
+    main, side = model.current, Stream(model, "side")
+    model.current = side
+    aside = side.op("input of the second request")
+    _submit(srv, serve.SEG_SUM)
+    model.current = main
+    late = main.op("queued between submit and run")
+    n0 = len(model.ops)
+    srv.run()
+    queued = model.ops[n0:]
+    assert {w for w, _, _ in queued} >= {"tcu_copy_async", "tcu_pack"}
+    for what, s, before in queued:
+        assert {early, aside, late} <= before, what
+
+
+def test_release_keeps_the_readers_of_results_ahead(model):
+    """After release() a block may be overwritten: the kernels that read the results queued before come first."""
+    from tcuscan_b200 import serve
+
+    srv = _server(model)
+    r = _submit(srv, serve.SCAN)[0]
+    srv.run()
+    assert srv.result(r).numel() == 5000
+    main, side = model.current, Stream(model, "side")
+    model.current = side
+    reader = side.op("reads the result")
+    srv.release()
+    model.current = main
+    _submit(srv, serve.SCAN, k=3)
+    n0 = len(model.ops)
+    srv.run()
+    assert len(model.ops) > n0 and all(reader in before for _, _, before in model.ops[n0:])
