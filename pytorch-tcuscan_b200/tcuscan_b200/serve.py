@@ -199,9 +199,10 @@ class Server:
         self._keepalive = {}
 
     def __del__(self):
-        # the slots' streams may still read the pinned tables and the arena
-        for si in list(getattr(self, "inflight", ())):
-            self.slots[si].event.synchronize()
+        # the slots' streams may still read the pinned tables and the arena,
+        # and PyTorch does not see their copies (tcu_copy_async)
+        for sl in getattr(self, "slots", ()):
+            sl.stream.synchronize()
 
     # ---------------------------------------------------------------- table
     def _alloc(self, cap):
@@ -405,6 +406,9 @@ class Server:
             self.finished[b.id] = b
         else:
             self._free(b)
+        self._forget(ids)
+
+    def _forget(self, ids):
         if self._keepalive:
             for i in ids:
                 self._keepalive.pop(int(i), None)
@@ -449,10 +453,6 @@ class Server:
 
     # -------------------------------------------------------------- launch
     def _launch(self, cls, ids, nbytes):
-        op = int(self.op[ids[0]])
-        dti = int(self.dt[ids[0]])
-        dtype = DTYPES[dti]
-        eb = int(_EB[dti])
         si = self.free_slots.popleft()
         sl = self.slots[si]
         off, nbytes = self.arena.alloc(nbytes)
@@ -461,6 +461,29 @@ class Server:
         self.used += nbytes
         self.peak_used = max(self.peak_used, self.used)
         self.admit[ids] = self.now()
+        try:
+            b = self._queue(sl, ids, off, nbytes)
+        except BaseException:
+            # what was queued before the failure still uses the block and the
+            # tables, and may have left the workspace between use and clearing
+            _lib.lib.tcu_workspace_init(sl.ws.data_ptr(), sl.wsb, ctypes.c_void_p(sl.stream.cuda_stream))
+            sl.stream.synchronize()
+            self.arena.release(off, nbytes)
+            self.used -= nbytes
+            self.free_slots.append(si)
+            self._forget(ids)
+            raise
+        b.id, b.cls, b.ids, b.slot, b.off, b.bytes = self.batches, cls, ids, si, off, nbytes
+        self.bid[ids] = self.batches
+        self.batches += 1
+        self.inflight[si] = b
+
+    def _queue(self, sl, ids, off, nbytes):
+        """Lay a batch out in its block and queue its copies and kernels on the slot's stream."""
+        op = int(self.op[ids[0]])
+        dti = int(self.dt[ids[0]])
+        dtype = DTYPES[dti]
+        eb = int(_EB[dti])
         # requests read in place (large scan / seg_sum inputs, 16-byte aligned)
         # and the rest, which are packed back to back
         solo = np.zeros(ids.size, dtype=bool)
@@ -496,13 +519,6 @@ class Server:
         else:
             meta.append(dst.view(np.uint8))
         mb = max(sum(m.size for m in meta), 16)
-        if mb > sl.pinned.numel():
-            sl.pinned = torch.empty(_roundup(mb, 1 << 20), dtype=torch.uint8, pin_memory=True)
-        pn = sl.pinned.numpy()
-        o = 0
-        for m in meta:
-            pn[o:o + m.size] = m
-            o += m.size
 
         # buffers of the block: [meta | x | outputs ...]
         cur = [off]
@@ -514,6 +530,32 @@ class Server:
 
         m_off = carve(mb)
         x_off = carve(total * eb)
+        out_dtype = dtype if op == COMPRESS else tcuscan_ops._scan_out_dtype(dtype)
+        if op == SCAN:
+            npad_s = _roundup(self.n[ids_s], ALIGN)
+            out_len = total + int(npad_s.sum())
+            z_off = carve(out_len * 4)
+        elif op == SEG_SUM:
+            nbt = int(nb.sum()) if k else 0
+            out_p = max(nbt - 1, 0)
+            b_off = carve(nbt * 8)
+            out_len = max(out_p + int(self.nseg[ids_s].sum()), 1)
+            z_off = carve(out_len * 4)
+        else:
+            mk_off = carve(total)
+            z_off = carve(total * eb)
+            p_off = carve((k + 1) * 8)
+            out_len = total
+        if cur[0] - off > nbytes:
+            raise AssertionError("batch layout overruns its block")
+
+        if mb > sl.pinned.numel():
+            sl.pinned = torch.empty(_roundup(mb, 1 << 20), dtype=torch.uint8, pin_memory=True)
+        pn = sl.pinned.numpy()
+        o = 0
+        for m in meta:
+            pn[o:o + m.size] = m
+            o += m.size
         base = self.arena.base
         st = sl.stream
         sp = ctypes.c_void_p(st.cuda_stream)
@@ -529,9 +571,6 @@ class Server:
                 tcuscan_ops.check(L.tcu_copy_async(base + m_off, sl.pinned.data_ptr(), mb, sp), "serve request table")
                 tcuscan_ops.check(L.tcu_pack(base + m_off, k, eb, eb, base + x_off, total, sp), "serve pack")
             if op == SCAN:
-                out_dtype = tcuscan_ops._scan_out_dtype(dtype)
-                npad_s = _roundup(self.n[ids_s], ALIGN)
-                z_off = carve((total + int(npad_s.sum())) * 4)
                 if k:
                     s_ = L.tcu_seg_bounds(base + x_off, _lib.DTYPE_CODE[dtype], total, S, base + m_off + items.nbytes,
                                           _lib.TCU_INT64, k, 0, base + z_off, wsp, sl.wsb, sp)
@@ -546,14 +585,8 @@ class Server:
                     tcuscan_ops.check(s_, "serve scan (in place)")
                     self.roff[r], self.rlen[r] = o_, nr
                     o_ += int(npad_s[j])
-                out_len = max(o_, 1)
             elif op == SEG_SUM:
-                out_dtype = tcuscan_ops._scan_out_dtype(dtype)
                 iw = int(self.iw[ids[0]])
-                nbt = int(nb.sum()) if k else 0
-                b_off = carve(nbt * 8)
-                out_p = max(nbt - 1, 0)
-                z_off = carve(max(out_p + int(self.nseg[ids_s].sum()), 1) * 4)
                 if k:
                     tcuscan_ops.check(L.tcu_pack(base + m_off + items.nbytes, k, iw, 8, base + b_off, nbt, sp),
                                       "serve pack row pointers")
@@ -575,12 +608,7 @@ class Server:
                         tcuscan_ops.check(s_, "serve seg_sum (in place)")
                     self.roff[r], self.rlen[r] = o_, ns
                     o_ += ns
-                out_len = max(o_, 1)
             else:
-                out_dtype = dtype
-                mk_off = carve(total)
-                z_off = carve(total * eb)
-                p_off = carve((k + 1) * 8)
                 tcuscan_ops.check(L.tcu_pack(base + m_off + items.nbytes, k, 1, 1, base + mk_off, total, sp),
                                   "serve pack masks")
                 starts = base + m_off + 2 * items.nbytes
@@ -589,16 +617,10 @@ class Server:
                 tcuscan_ops.check(s_, "serve compress")
                 tcuscan_ops.check(L.tcu_copy_async(sl.pos_host.data_ptr(), base + p_off, (k + 1) * 8, sp),
                                   "serve compress positions")
-                out_len = total
             sl.event.record(st)
-        if cur[0] - off > nbytes:
-            raise AssertionError("batch layout overran its block")
         b = _Batch()
-        b.id, b.cls, b.ids, b.slot, b.off, b.bytes = self.batches, cls, ids, si, off, nbytes
         b.out_off, b.out_dtype, b.out_len, b.out = z_off, out_dtype, out_len, None
-        self.bid[ids] = self.batches
-        self.batches += 1
-        self.inflight[si] = b
+        return b
 
     # ------------------------------------------------------------- results
     def result(self, rid):

@@ -50,8 +50,9 @@ class Event:
         self.point = (stream or self.model.current).before
 
     def query(self):
-        self.model.done |= self.point
-        return True
+        if not self.model.busy:
+            self.model.done |= self.point
+        return not self.model.busy
 
     def synchronize(self):
         self.model.done |= self.point
@@ -61,7 +62,7 @@ class Model:
     """Streams, and a C interface whose calls only queue operations."""
 
     def __init__(self):
-        self.ops, self.streams, self.done, self.fail = [], {}, frozenset(), None
+        self.ops, self.streams, self.done, self.fail, self.busy = [], {}, frozenset(), None, False
         self.current = Stream(self, "caller")
 
     def __getattr__(self, name):  # lib.tcu_*
@@ -195,3 +196,56 @@ def test_release_keeps_the_readers_of_results_ahead(model):
     n0 = len(model.ops)
     srv.run()
     assert len(model.ops) > n0 and all(reader in before for _, _, before in model.ops[n0:])
+
+
+@pytest.mark.parametrize("op,fails", [(0, "tcu_seg_bounds"), (1, "tcu_pack"), (2, "tcu_compress_segments")])
+def test_a_launch_that_fails_half_way_gives_everything_back(model, op, fails):
+    """The copies and kernels queued before the failing call have ended before the error leaves the loop (the
+    batch is not registered anywhere); the slot and the block are free again and serve the next batch."""
+    from tcuscan_b200 import serve
+    from tcuscan_ops import TcuError
+
+    srv = _server(model)
+    whole = list(srv.arena.free)
+    _submit(srv, op)
+    n0 = len(model.ops)
+    model.fail = fails
+    with pytest.raises(TcuError):
+        srv.run()
+    slot_ops = {i for i, (w, s, _) in enumerate(model.ops) if i >= n0 and s.name == "slot"}
+    assert slot_ops and slot_ops <= model.done
+    assert srv.used == 0 and srv.arena.free == whole
+    assert sorted(srv.free_slots) == [0, 1] and not srv.inflight
+    model.fail = None
+    r = _submit(srv, op)[0]
+    srv.run()
+    srv.result(r)
+
+
+def test_an_undersized_block_is_seen_before_anything_is_queued(model, monkeypatch):
+    from tcuscan_b200 import serve
+
+    srv = _server(model)
+    whole = list(srv.arena.free)
+    _submit(srv, serve.SCAN)
+    monkeypatch.setattr(srv, "_take", lambda cls, room, take=srv._take: (take(cls, room)[0], 4096))
+    n0 = len(model.ops)
+    with pytest.raises(AssertionError):
+        srv.run()
+    assert {w for w, _, _ in model.ops[n0:]} <= {"tcu_workspace_init"}  # the slot's workspace, not the block
+    assert srv.arena.free == whole and len(srv.free_slots) == 2
+
+
+def test_a_server_that_goes_away_waits_for_its_streams(model):
+    """PyTorch does not see the copies from the pinned tables: they have ended before the tables, the workspaces
+    and the arena go back to their allocators -- also those of a batch that no list holds."""
+    from tcuscan_b200 import serve
+
+    srv = _server(model)
+    _submit(srv, serve.COMPRESS)
+    model.busy = True
+    srv.step()
+    srv.slots[1].stream.op("a copy that nothing registered")
+    srv.__del__()
+    assert {i for i, (w, s, _) in enumerate(model.ops) if s.name == "slot"} <= model.done
+    serve.Server.__del__(object.__new__(serve.Server))  # a constructor that raised
