@@ -13,6 +13,7 @@
 #include <stdint.h>
 
 #include <climits>
+#include <cstddef>
 
 #include "tcuscan.h"
 
@@ -33,6 +34,7 @@ struct WsHeader {
   uint32_t pad[10];
 };
 static_assert(sizeof(WsHeader) == 64, "header size");
+static_assert(offsetof(WsHeader, error) == 12, "the serving loop copies the three error words from here");
 
 // Look-back descriptor states: bits[1:0] state, bit 2 = the tile contains a
 // segment start (its aggregate is already a complete carry), bits[31:3] =

@@ -32,7 +32,9 @@ its stream.  This module keeps the device busy with many requests at once:
   kernels that fill a request's inputs, and those that read results whose
   blocks are used again.
 - Completion is read from one CUDA event per slot (polled, never a device
-  synchronisation).  A request's result is a view of its batch's block.
+  synchronisation).  A request's result is a view of its batch's block.  A
+  batch in which a bounded device wait ran out raises TcuError from the loop
+  and has no results.
 
 Every request's result equals what the single call returns for it: integer
 results bit for bit, floating results within the scan family's tolerance
@@ -65,6 +67,7 @@ ALIGN = 256        # elements: every request starts on a 256-element boundary of
 # 2.39, 2^22 2.54 and 2^23 2.55 TB/s.
 SOLO_MIN = 1 << 22
 BLOCK_ALIGN = 256  # bytes: arena blocks and the buffers inside them
+WS_ERROR = 12  # offset of the workspace header's error, err_site and err_chunk words
 BATCH_SLACK = 8192  # bytes per batch for buffer alignment inside its block
 
 # matches tcu_pack_item_t (include/tcuscan.h)
@@ -117,7 +120,7 @@ class Arena:
 
 
 class _Slot:
-    __slots__ = ("idx", "stream", "event", "pinned", "pos_host", "ws", "wsb", "seen")
+    __slots__ = ("idx", "stream", "event", "pinned", "pos_host", "err_host", "ws", "wsb", "seen")
 
 
 class _Batch:
@@ -172,6 +175,7 @@ class Server:
             sl.event = torch.cuda.Event(enable_timing=self.timing)
             sl.pinned = torch.empty(1 << 20, dtype=torch.uint8, pin_memory=True)
             sl.pos_host = torch.empty(max_batch + 1, dtype=torch.int64, pin_memory=True)
+            sl.err_host = torch.empty(3, dtype=torch.int32, pin_memory=True)
             sl.ws = torch.empty(ws_need, dtype=torch.uint8, device=self.dev)  # owned by the slot
             sl.wsb = ctypes.c_size_t(ws_need)
             sl.seen = 0
@@ -394,6 +398,13 @@ class Server:
         t = self.now()
         ids = b.ids
         sl = self.slots[b.slot]
+        code, site, chunk = sl.err_host.tolist()
+        if code:  # a wait in the batch ran out: no result of it is right
+            _lib.lib.tcu_workspace_init(sl.ws.data_ptr(), sl.wsb, ctypes.c_void_p(sl.stream.cuda_stream))
+            self.free_slots.append(b.slot)
+            self._free(b)
+            self._forget(ids)
+            raise tcuscan_ops.TcuError(code, "serve batch", f"site {site}, chunk {chunk}")
         self.done[ids] = t
         if self.timing and self.start_event is not None:
             self.done_gpu[ids] = self.start_event.elapsed_time(sl.event) * 1e-3
@@ -617,6 +628,7 @@ class Server:
                 tcuscan_ops.check(s_, "serve compress")
                 tcuscan_ops.check(L.tcu_copy_async(sl.pos_host.data_ptr(), base + p_off, (k + 1) * 8, sp),
                                   "serve compress positions")
+            tcuscan_ops.check(L.tcu_copy_async(sl.err_host.data_ptr(), wsp + WS_ERROR, 12, sp), "serve error words")
             sl.event.record(st)
         b = _Batch()
         b.out_off, b.out_dtype, b.out_len, b.out = z_off, out_dtype, out_len, None

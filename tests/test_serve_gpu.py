@@ -358,3 +358,25 @@ def test_requests_still_being_written_when_they_are_served():
         assert torch.equal(got[2], torch.cumsum(want[: 1 << 20].long() + 1, 0).int())
         assert all(torch.equal(srv.result(i), torch.cumsum(base.long(), 0).int()) for i in z)
         srv.release()
+
+
+def test_server_raises_a_batch_whose_wait_ran_out():
+    """The library's self-test leaves a timed-out wait in a slot's workspace (1 ms, no fault): the batch served
+    from that slot is refused with the error, and the next one is right."""
+    from tcuscan_b200 import serve
+
+    L = _lib()
+    x = torch.randint(-8, 9, (100_000,), dtype=torch.int8, device=DEV)
+    srv = serve.Server(DEV, budget_bytes=1 << 30, slots=1, keep_results=True)
+    sl = srv.slots[0]
+    assert L.lib.tcu_selftest_wait_timeout(1, 1_000_000, sl.ws.data_ptr(), sl.wsb,
+                                           ctypes.c_void_p(sl.stream.cuda_stream)) == 0
+    r = srv.submit("scan", x)
+    with pytest.raises(L.TcuError, match="timed out"):
+        srv.run()
+    with pytest.raises(RuntimeError):
+        srv.result(r)
+    r = srv.submit("scan", x)
+    srv.run()
+    assert torch.equal(srv.result(r), torch.cumsum(x.long(), 0).int())
+    assert srv.used == srv.finished[int(srv.bid[r])].bytes

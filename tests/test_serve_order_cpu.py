@@ -9,6 +9,7 @@ before must be in the set of every operation that reads or overwrites the same
 memory.
 """
 import contextlib
+import ctypes
 import types
 
 import numpy as np
@@ -63,6 +64,7 @@ class Model:
 
     def __init__(self):
         self.ops, self.streams, self.done, self.fail, self.busy = [], {}, frozenset(), None, False
+        self.error = (0, 0, 0)
         self.current = Stream(self, "caller")
 
     def __getattr__(self, name):  # lib.tcu_*
@@ -74,6 +76,8 @@ class Model:
                 return 1 << 12
             if name == self.fail:
                 return 3  # TCU_ERR_LAUNCH
+            if name == "tcu_copy_async" and args[2] == 12:  # the slot's error words
+                ctypes.memmove(args[0], (ctypes.c_uint32 * 3)(*self.error), 12)
             self.streams[args[-1].value].op(name)
             return 0
 
@@ -249,3 +253,25 @@ def test_a_server_that_goes_away_waits_for_its_streams(model):
     srv.__del__()
     assert {i for i, (w, s, _) in enumerate(model.ops) if s.name == "slot"} <= model.done
     serve.Server.__del__(object.__new__(serve.Server))  # a constructor that raised
+
+
+@pytest.mark.parametrize("op", [0, 1, 2])
+def test_a_device_error_is_raised_instead_of_results(model, op):
+    """A bounded wait that ran out is recorded in the slot's workspace: the loop raises it, hands out nothing of
+    the batch, and serves on with the slot's workspace reset."""
+    from tcuscan_ops import TcuError
+
+    srv = _server(model)
+    whole = list(srv.arena.free)
+    r = _submit(srv, op)[0]
+    model.error = (4, 100, 7)
+    with pytest.raises(TcuError, match="site 100, chunk 7"):
+        srv.run()
+    with pytest.raises(RuntimeError):
+        srv.result(r)
+    assert srv.arena.free == whole and srv.used == 0 and len(srv.free_slots) == 2 and not srv.inflight
+    assert [s.name for _, s, _ in model.find("tcu_workspace_init")][2:] == ["slot"]
+    model.error = (0, 0, 0)
+    r = _submit(srv, op)[0]
+    srv.run()
+    srv.result(r)
