@@ -235,18 +235,15 @@ tcu_status_t launch_block_tc(const void* x, int64_t n, const void* upper, const 
   tcu_status_t s = make_map_2d(&in_map, x, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, S, (uint64_t)rows, 64, 128);
   if (s != TCU_OK) return s;
   auto kern = block_scan_tc_kernel<S>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_LAUNCH);
-    if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(block_scan_tc)");
-    attr_set = true;
-  }
+  static DeviceSet opted;
+  cudaError_t e = allow_smem(opted, C::SMEM_LAUNCH, kern);
+  if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(block_scan_tc)");
   int64_t grid = (int64_t)sm_count() * 2;
   if (nblocks < grid) grid = nblocks;
   kern<<<(unsigned)grid, kBtThreads, C::SMEM_LAUNCH, st>>>(in_map, static_cast<const __half*>(upper),
                                                            static_cast<const __half*>(lower), static_cast<float*>(z),
                                                            rows, nblocks, static_cast<WsHeader*>(ws), timeout_ns());
-  cudaError_t e = cudaGetLastError();
+  e = cudaGetLastError();
   return e == cudaSuccess ? TCU_OK : cuda_fail(e, "block_scan_tc launch");
 }
 

@@ -249,16 +249,13 @@ static tcu_status_t launch_scan_tc(const void* x, int64_t n, void* z, double sta
   }
   const int smem = C::SMEM_BYTES < 120 * 1024 ? 120 * 1024 : C::SMEM_BYTES;
   auto kern = scan_tc_kernel<InT, W, MODE>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute");
-    attr_set = true;
-  }
+  static DeviceSet opted;
+  cudaError_t e = allow_smem(opted, smem, kern);
+  if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute");
   int grid = grid_ctas();
   if (p.num_tiles < grid) grid = (int)p.num_tiles;
   kern<<<grid, C::THREADS, smem, st>>>(in_map, out_map, p);
-  cudaError_t e = cudaGetLastError();
+  e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "scan_tc_kernel launch");
   if (tile_first) {
     e = cudaMemsetAsync(tile_first, 0, (size_t)p.num_tiles * sizeof(long long), st);

@@ -565,16 +565,13 @@ template <int EB, int IDX, int IB, bool SPLIT, bool BITS>
 static tcu_status_t launch_compact(const CompactParams& p, cudaStream_t st) {
   using C = CmpCfg<EB, IDX, IB>;
   auto kern = compact_kernel<EB, IDX, IB, SPLIT, BITS>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
-    if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(compress)");
-    attr_set = true;
-  }
+  static DeviceSet opted;
+  cudaError_t e = allow_smem(opted, C::SMEM, kern);
+  if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(compress)");
   const int64_t ctas = ((p.n + kCmpTile - 1) / kCmpTile + kCmpWarps - 1) / kCmpWarps;
   if (ctas > 0x7FFFFFFF) return TCU_ERR_ARG;
   kern<<<(unsigned)ctas, kCmpThreads, C::SMEM, st>>>(p);
-  cudaError_t e = cudaGetLastError();
+  e = cudaGetLastError();
   return e == cudaSuccess ? TCU_OK : cuda_fail(e, "compact_kernel launch");
 }
 

@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include "tcu_lookback.cuh"
+#include "tcu_smem.h"
 #include "tcuscan.h"
 
 namespace tcu {

@@ -431,16 +431,10 @@ template <typename K, int CODEC, bool FIRST, bool LAST>
 static cudaError_t launch_scatter(bool async_ok, int C, cudaStream_t st, const K* src_k, const int* src_i, K* dk, int* di,
                                   const int* base, int64_t n, int shift, int64_t T) {
   constexpr int smem = ScatterSmem<K>::BYTES;
-  static bool attr = false;
-  if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(rs_scatter_kernel<K, CODEC, FIRST, LAST, true>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(rs_scatter_kernel<K, CODEC, FIRST, LAST, false>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-    attr = true;
-  }
+  static DeviceSet opted;
+  cudaError_t e = allow_smem(opted, smem, rs_scatter_kernel<K, CODEC, FIRST, LAST, true>,
+                             rs_scatter_kernel<K, CODEC, FIRST, LAST, false>);
+  if (e != cudaSuccess) return e;
   if (async_ok)
     rs_scatter_kernel<K, CODEC, FIRST, LAST, true><<<C, kRsThreads, smem, st>>>(src_k, src_i, dk, di, base, n, shift, T);
   else

@@ -771,19 +771,9 @@ static TopkPlan tk_plan(int64_t n, int64_t k) {
 }
 
 template <int CODEC, bool VEC>
-static cudaError_t tk_hist_attr() {
-  static bool done = false;
-  if (done) return cudaSuccess;
-  cudaError_t e = cudaFuncSetAttribute(topk_hist_kernel<CODEC, 0, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, 65536);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(topk_hist_kernel<CODEC, 1, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, 65536);
-  done = e == cudaSuccess;
-  return e;
-}
-
-template <int CODEC, bool VEC>
 static tcu_status_t topk_run(TopkParams p, const TopkPlan& t, cudaStream_t st) {
-  cudaError_t e = tk_hist_attr<CODEC, VEC>();
+  static DeviceSet opted;
+  cudaError_t e = allow_smem(opted, 65536, topk_hist_kernel<CODEC, 0, VEC>, topk_hist_kernel<CODEC, 1, VEC>);
   if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(topk)");
   e = cudaMemsetAsync(p.st, 0, kTkHead, st);
   if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync(topk state)");
@@ -802,14 +792,11 @@ static tcu_status_t topk_run(TopkParams p, const TopkPlan& t, cudaStream_t st) {
 template <int CODEC, bool VEC>
 static tcu_status_t topk_small(const uint16_t* x, int n, int k, uint16_t* out, int* idx_out, cudaStream_t st) {
   constexpr int smem = kTkSmallThreads * 256;
-  static bool attr = false;
-  if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(topk_small_kernel<CODEC, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(topk)");
-    attr = true;
-  }
+  static DeviceSet opted;
+  cudaError_t e = allow_smem(opted, smem, topk_small_kernel<CODEC, VEC>);
+  if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(topk)");
   topk_small_kernel<CODEC, VEC><<<1, kTkSmallThreads, smem, st>>>(x, n, k, out, idx_out);
-  cudaError_t e = cudaGetLastError();
+  e = cudaGetLastError();
   return e == cudaSuccess ? TCU_OK : cuda_fail(e, "topk launch");
 }
 

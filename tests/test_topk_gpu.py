@@ -42,3 +42,24 @@ def test_topk_forms(kind, n):
         rv, ri = oracle.topk(x.numpy(), k)
         assert np.array_equal(i.cpu().numpy(), ri), (k, "positions")
         assert np.array_equal(v.cpu().numpy().view(np.uint16), rv.view(np.uint16)), (k, "values")
+
+
+@pytest.mark.skipif(torch.cuda.device_count() < 2, reason="needs two GPUs in one process")
+def test_every_device_of_a_process():
+    """Kernels with more than 48 KB of shared memory on the second GPU after the first."""
+    import tcuscan_ops
+
+    x = _input("normal", 1_500_007)
+    m = (x > 0).to(torch.int8)
+    for dev in ("cuda:0", "cuda:1"):
+        with torch.cuda.device(dev):
+            for n in (30_000, x.numel()):
+                v, i = tcuscan_ops.run_topk_fp16(x[:n].to(dev), 100, 0, 0, 64)
+                rv, ri = oracle.topk(x[:n].numpy(), 100)
+                assert np.array_equal(i.cpu().numpy(), ri) and np.array_equal(v.cpu().numpy(), rv)
+            v, i = tcuscan_ops.run_compress_ind_no_arange(x.float().to(dev), m.to(dev), 64)
+            assert np.array_equal(i.cpu().numpy(), np.nonzero(m.numpy())[0])
+            s, _ = tcuscan_ops.run_radix_sort(x.to(dev), 128)
+            assert torch.equal(s.cpu(), torch.sort(x).values)
+            z = tcuscan_ops.run_scan_multi_core(m.to(dev).repeat(4), 64)
+            assert torch.equal(z.cpu(), torch.cumsum(m.repeat(4).long(), 0).int())
