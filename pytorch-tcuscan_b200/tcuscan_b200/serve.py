@@ -73,6 +73,10 @@ BATCH_SLACK = 8192  # bytes per batch for buffer alignment inside its block
 # matches tcu_pack_item_t (include/tcuscan.h)
 PACK_ITEM = np.dtype([("src", "<u8"), ("dst", "<i8"), ("n", "<i8"), ("len", "<i8"), ("add", "<i8")])
 
+# block bytes of a request, by op: per padded element (and dtype), per row, and once
+_ELEM_BYTES = np.stack([_EB + 4, _EB, 1 + 2 * _EB])  # x and scan; x; mask, x and output
+_ROW_BYTES = np.array([0, 8 + 4, 0])                 # row pointer and sum
+_REQUEST_BYTES = 2 * PACK_ITEM.itemsize + 16 + np.array([0, 8 + 4, 8])  # request table; last row pointer; position
 
 _HERE = contextlib.nullcontext()
 
@@ -318,26 +322,9 @@ class Server:
     def _bytes(self, ids):
         """Block bytes each request adds to its batch (inputs, outputs, row
         pointers and its entries of the batch's request table)."""
-        npad = _roundup(self.n[ids], ALIGN)
-        eb = _EB[self.dt[ids]]
         op = self.op[ids]
-        b = npad * eb + 2 * PACK_ITEM.itemsize + 16
-        b = b + np.where(op == SCAN, npad * 4, 0)
-        b = b + np.where(op == SEG_SUM, (self.nseg[ids] + 1) * 12, 0)
-        b = b + np.where(op == COMPRESS, npad * (1 + eb) + 8, 0)
-        return b
-
-    def _class_bytes(self, ids):
-        """_bytes of requests of one class (op and dtype of the first)."""
         npad = _roundup(self.n[ids], ALIGN)
-        i = ids[0]
-        eb, op = int(_EB[self.dt[i]]), int(self.op[i])
-        fixed = 2 * PACK_ITEM.itemsize + 16
-        if op == SCAN:
-            return npad * (eb + 4) + fixed
-        if op == SEG_SUM:
-            return npad * eb + (self.nseg[ids] + 1) * 12 + fixed
-        return npad * (1 + 2 * eb) + (fixed + 8)
+        return npad * _ELEM_BYTES[op, self.dt[ids]] + self.nseg[ids] * _ROW_BYTES[op] + _REQUEST_BYTES[op]
 
     # ---------------------------------------------------------------- loop
     def _arrivals(self):
@@ -365,7 +352,7 @@ class Server:
         room -= BATCH_SLACK
         while q and count < self.max_batch:
             ids = q[0]
-            b = self._class_bytes(ids)  # a queue holds one class
+            b = self._bytes(ids)
             cum = np.cumsum(b)
             k = int(np.searchsorted(cum, room - used, side="right"))
             k = min(k, self.max_batch - count)

@@ -129,12 +129,12 @@ def _server(m, **kw):
     return serve.Server("cuda:0", budget_bytes=4 << 20, slots=2, keep_results=True, **kw)
 
 
-def _submit(srv, op, n=5000, k=1):
-    """k int8 requests on memory of nobody's (the model reads nothing)."""
-    nseg = 40 if op == 1 else 0
-    return srv.submit_many(np.full(k, op, np.int8), np.zeros(k, np.int8), np.full(k, n), np.full(k, 4096, np.uint64),
-                           np.full(k, 8192, np.uint64), np.full(k, nseg), np.full(k, 4 if op == 1 else 0, np.int8),
-                           np.full(k, srv.now()))
+def _submit(srv, op, n=5000, k=1, dt=0, nseg=40, iw=4):
+    """k requests (int8 unless dt says otherwise) on memory of nobody's (the model reads nothing)."""
+    n = np.broadcast_to(n, k)
+    return srv.submit_many(np.full(k, op, np.int8), np.full(k, dt, np.int8), n, np.full(k, 4096, np.uint64),
+                           np.full(k, 8192, np.uint64), np.broadcast_to(nseg if op == 1 else 0, k),
+                           np.full(k, iw if op == 1 else 0, np.int8), np.full(k, srv.now()))
 
 
 def test_construction_follows_the_callers_work(model):
@@ -275,3 +275,22 @@ def test_a_device_error_is_raised_instead_of_results(model, op):
     r = _submit(srv, op)[0]
     srv.run()
     srv.result(r)
+
+
+@pytest.mark.parametrize("op,iw", [(0, 0), (1, 4), (1, 8), (2, 0)])
+@pytest.mark.parametrize("dt", [0, 1, 2])
+def test_blocks_hold_what_the_batches_lay_out(model, monkeypatch, op, iw, dt):
+    """Admission sizes a block before the launch lays it out (and refuses one that is too small): every op, dtype
+    and row-pointer width, requests of every length, packed and in place, with no more slack than the rounding of
+    the block's buffers (at most six) to BLOCK_ALIGN takes."""
+    from tcuscan_b200 import serve
+
+    rng = np.random.default_rng(100 * op + 10 * iw + dt)
+    monkeypatch.setattr(serve, "SOLO_MIN", 1 << 12)
+    monkeypatch.setattr(serve, "BATCH_SLACK", 6 * serve.BLOCK_ALIGN)
+    srv = serve.Server("cuda:0", budget_bytes=64 << 20, slots=2)
+    for k in (1, 1, 2, 7, 40, 300):
+        n = np.exp(rng.uniform(0, np.log(9000), size=k)).astype(np.int64)
+        _submit(srv, op, n, k, dt, nseg=rng.integers(0, 400, size=k), iw=iw)
+        srv.run()
+    assert srv.used == 0 and np.isfinite(srv.done[: srv._n]).all()
