@@ -322,7 +322,8 @@ __device__ __forceinline__ uint32_t tk_sample_rank(const uint32_t (&key)[4], int
   return hi;
 }
 
-__device__ __forceinline__ uint32_t tk_hash(uint32_t v) {  // an integer mix with full avalanche
+// The published integer hash "lowbias32" (C. Wellons, hash-prospector).
+__device__ __forceinline__ uint32_t tk_hash(uint32_t v) {
   v ^= v >> 16;
   v *= 0x7FEB352Du;
   v ^= v >> 15;
