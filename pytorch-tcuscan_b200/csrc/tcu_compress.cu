@@ -76,7 +76,7 @@ struct CompactParams {
 // A warp takes its tile in parts of SUB elements: U vectors of 16 bytes per
 // lane, as many as fit the staging area and, with gathered indices, about 10
 // vectors of values and indices in registers.
-template <int EB, int IDX, int IB>
+template <int EB, int IDX, int IB, bool SPLIT>
 struct CmpCfg {
   static constexpr int EPV = 16 / EB;  // elements of a vector
   static constexpr int IBX = IDX ? IB : 0;
@@ -93,10 +93,15 @@ struct CmpCfg {
   static constexpr int X_BYTES = SUB * EB + 64;
   static constexpr int I_BYTES = IBX ? SUB * IBX + 64 : 0;
   static constexpr int SMEM = kCmpWarps * (X_BYTES + I_BYTES);
-  // Values alone run faster with 64 registers and four CTAs per SM (fp32
-  // 2^28: 328 -> 288 us), one-byte values (162 -> 172 us) and most forms with
-  // indices (fp32 positions: 395 -> 450 us) with the registers they ask for.
-  static constexpr int MIN_CTAS = IDX == 0 && EB >= 2 ? 4 : 0;  // 0: no bound
+  // Values alone run faster with 64 registers and four CTAs per SM than with
+  // the 63 to 109 they ask for, spills of up to 100 bytes included (512 MB of
+  // values, mask 0.3, the compaction kernel alone): 2 bytes 131 against 135 us
+  // and split 203 against 213, 4 bytes 109 against 128 and split 179 against
+  // 193, 8 bytes 107 against 110; at mask 0.9 195 against 194, 160 against 176
+  // and 163 against 162.  The 8-byte split does not (183 against 173 us), nor
+  // do one-byte values (162 -> 172 us for a whole call) and most forms with
+  // indices (fp32 positions: 395 -> 450 us): they take the registers they ask for.
+  static constexpr int MIN_CTAS = IDX == 0 && EB >= 2 && !(EB == 8 && SPLIT) ? 4 : 0;  // 0: no bound
   static_assert(kCmpTile % SUB == 0, "parts of a tile");
 };
 
@@ -204,8 +209,8 @@ __device__ __forceinline__ void push_if(uint32_t b, uint32_t bit, uint32_t& addr
 // others after all selected ones (at total + the unselected elements before
 // them), so a part writes two runs.  Bound by HBM: see the file comment.
 template <int EB, int IDX, int IB, bool SPLIT, bool BITS>
-__global__ void __launch_bounds__(kCmpThreads, (CmpCfg<EB, IDX, IB>::MIN_CTAS)) compact_kernel(const CompactParams p) {
-  using C = CmpCfg<EB, IDX, IB>;
+__global__ void __launch_bounds__(kCmpThreads, (CmpCfg<EB, IDX, IB, SPLIT>::MIN_CTAS)) compact_kernel(const CompactParams p) {
+  using C = CmpCfg<EB, IDX, IB, SPLIT>;
   using T = typename ElemT<EB>::T;
   using I = typename ElemT<(IB > 0 ? IB : 4)>::T;
   constexpr int EPV = C::EPV, U = C::U, SUB = C::SUB, V = 16 / EB, VI = 16 / (int)sizeof(I);
@@ -563,7 +568,7 @@ static tcu_status_t cmp_count(const int8_t* mask, int64_t n, const CmpScratch& s
 
 template <int EB, int IDX, int IB, bool SPLIT, bool BITS>
 static tcu_status_t launch_compact(const CompactParams& p, cudaStream_t st) {
-  using C = CmpCfg<EB, IDX, IB>;
+  using C = CmpCfg<EB, IDX, IB, SPLIT>;
   auto kern = compact_kernel<EB, IDX, IB, SPLIT, BITS>;
   static DeviceSet opted;
   cudaError_t e = allow_smem(opted, C::SMEM, kern);
