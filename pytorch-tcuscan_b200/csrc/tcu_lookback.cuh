@@ -132,9 +132,10 @@ struct LbScratch {
   uint32_t dmin[4];
 };
 
-// Warpgroup variant: the tile's aggregate was already published by another
-// warp; this publishes the inclusive prefix agg_inc + exclusive prefix.  The
-// first warp of the warpgroup looks back, one predecessor per lane per round
+// Warpgroup variant for full scans (no segment starts): the tile's aggregate
+// was already published by another warp; this publishes the inclusive prefix
+// agg_inc + exclusive prefix.  The first warp of the warpgroup looks back, one
+// predecessor per lane per round
 // (a 32-tile window), and hands the prefix to the other three warps through
 // `sc` at one named barrier.  Tiles finish nearly in order, so the nearest
 // inclusive prefix is normally a few tiles back: a 1024-tile window (eight
@@ -142,8 +143,7 @@ struct LbScratch {
 // scans, its extra loads and instructions landing on every tile.
 template <typename V>
 __device__ __forceinline__ V wg_lookback(int64_t tid, V agg_inc, V start, TileDesc* descs, uint32_t epoch,
-                                         const WaitCtx& wc, LbScratch* sc, int wg_thread, uint32_t bar_id,
-                                         int agg_seg = 0) {
+                                         const WaitCtx& wc, LbScratch* sc, int wg_thread, uint32_t bar_id) {
   if (tid == 0) return start;
   if (wg_thread < 32) {
     const int lane = wg_thread;
@@ -177,7 +177,7 @@ __device__ __forceinline__ V wg_lookback(int64_t tid, V agg_inc, V start, TileDe
           }
         }
         val = v_from_bits<V>(vb);
-        if ((f & 3u) == LB_INC || (f & LB_SEGSTART)) stop_d = (uint32_t)lane;
+        if ((f & 3u) == LB_INC) stop_d = (uint32_t)lane;
       }
       const uint32_t dmin = __reduce_min_sync(0xffffffffu, stop_d);
       acc += warp_sum_any(((uint32_t)lane <= dmin) ? val : V(0));
@@ -185,8 +185,7 @@ __device__ __forceinline__ V wg_lookback(int64_t tid, V agg_inc, V start, TileDe
       base -= 32;
     }
     if (lane == 0) {
-      desc_store(descs + tid, v_bits<V>(agg_seg ? agg_inc : acc + agg_inc),
-                 tag | (agg_seg ? LB_SEGSTART : 0u) | LB_INC);
+      desc_store(descs + tid, v_bits<V>(acc + agg_inc), tag | LB_INC);
       sc->sum[0] = v_bits<V>(acc);
     }
   }
@@ -198,10 +197,11 @@ __device__ __forceinline__ V wg_lookback(int64_t tid, V agg_inc, V start, TileDe
 
 // The same for the segmented modes, waiting only for the tiles up to the nearest
 // stop: a tile with a segment start publishes a complete carry while tiles behind
-// it are still to come (fp16 flag segmented scan of 2^26 elements 143 -> 134 us,
-// uneven fp32 rows 1.238 -> 1.224 ms).  Full scans, whose stops are inclusive
-// prefixes with every tile behind them published, keep the form above: 2^20 fp16
-// 10.45 against 10.52 us.
+// it are still to come (fp16 flag segmented scan of 2^26 elements 139 -> 132 us;
+// uneven fp32 rows and sorted bounds without a difference).  Full scans, whose
+// stops are inclusive prefixes with every tile behind them published, keep the
+// form above: 2^20 fp16 10.45 us against 10.52 with this one, and 10.30 since
+// it looks for no segment starts.
 template <typename V>
 __device__ __forceinline__ V wg_lookback_nearest(int64_t tid, V agg_inc, V start, TileDesc* descs, uint32_t epoch,
                                                  const WaitCtx& wc, LbScratch* sc, int wg_thread, uint32_t bar_id,
