@@ -85,8 +85,9 @@ TCU_API void tcu_set_phase_profile(int enable);
  * `ws` (read it with tcu_workspace_error) and returns.  Nothing faults. */
 TCU_API tcu_status_t tcu_selftest_wait_timeout(int which, uint64_t timeout_ns, void* ws, size_t ws_bytes,
                                                void* stream);
-/* Tuning: CTAs of the persistent scan and compaction launches (0 = one per
- * SM, the default; smaller values leave SMs to concurrent launches).
+/* Tuning: CTAs of the persistent scan launches (0 = one per SM, the default;
+ * smaller values leave SMs to concurrent launches).  The compaction is not
+ * persistent (one CTA per eight 2048-element tiles) and takes no cap.
  * Process-wide; the autotuner sets it per size class. */
 TCU_API void tcu_set_max_ctas(int n);
 TCU_API int tcu_get_max_ctas(void);

@@ -9,9 +9,10 @@ device by ``tune()``:
     scan      tcuscan_ops.run_scan_multi_core              S (int8: 32/64/128,
                                                            fp16: 16..128), CTAs
     seg       batched uneven rows (sorted segment starts)  S (32/64), CTAs
-    compress  tcuscan_ops.run_compress_pos                 CTAs
-              (the compaction takes a CTA per eight tiles whatever the cap, so its
-              entries record times only)
+
+The compaction has nothing to tune: it takes a CTA per eight tiles whatever the
+cap.  ``tune(ops=("compress",))`` still times run_compress_pos; no call looks
+such an entry up, and neither the defaults nor the shipped table hold any.
 
 Entries are keyed by op, dtype and floor(log2(n)); lookups use the nearest
 tuned size of the same op and dtype.  The table is JSON (``TCU_AUTOTUNE_CACHE``
@@ -157,7 +158,7 @@ def _workload(op, dtype, n, device):
     raise ValueError(op)
 
 
-def tune(device=None, ops=("scan", "seg", "compress"), dtypes=DTYPES, log2_sizes=(16, 20, 24, 28),
+def tune(device=None, ops=("scan", "seg"), dtypes=DTYPES, log2_sizes=(16, 20, 24, 28),
          cta_fracs=(1.0, 0.75, 0.5), steps=10, warmup=3, path=None, timer=None, workload=None, write=True):
     """Measure every (S, CTA count) candidate per op, dtype and size, keep the
     fastest, and write the table.  `timer(fn, steps, warmup) -> ms` and
@@ -206,7 +207,7 @@ if __name__ == "__main__":  # python -m tcuscan_b200.autotune [--out PATH] [--si
     ap = argparse.ArgumentParser(description="measure and write the tile-parameter table")
     ap.add_argument("--out", default=CACHE)
     ap.add_argument("--sizes", default="16,20,24,28")
-    ap.add_argument("--ops", default="scan,seg,compress")
+    ap.add_argument("--ops", default="scan,seg")
     a = ap.parse_args()
     t = tune(ops=tuple(a.ops.split(",")), log2_sizes=tuple(int(v) for v in a.sizes.split(",")), path=a.out)
     for k, v in sorted(t["entries"].items()):
