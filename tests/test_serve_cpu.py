@@ -128,3 +128,11 @@ def test_arena_first_fit_and_coalescing():
         a.release(*b)
     assert a.free == [(0, 1 << 20)] and a.largest() == 1 << 20
     assert a.alloc(2 << 20) == (None, 0)
+
+
+def test_copy_async_arguments():
+    from tcuscan_ops import _lib as L
+
+    assert L.lib.tcu_copy_async(None, None, 0, None) == L.TCU_OK  # nothing to copy
+    assert L.lib.tcu_copy_async(None, 4096, 8, None) == L.TCU_ERR_ARG
+    assert L.lib.tcu_copy_async(4096, None, 8, None) == L.TCU_ERR_ARG

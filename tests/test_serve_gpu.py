@@ -380,3 +380,38 @@ def test_server_raises_a_batch_whose_wait_ran_out():
     srv.run()
     assert torch.equal(srv.result(r), torch.cumsum(x.long(), 0).int())
     assert srv.used == srv.finished[int(srv.bid[r])].bytes
+
+
+def test_copy_async_every_direction():
+    L = _lib()
+    st = torch.cuda.Stream(DEV)
+    sp = ctypes.c_void_p(st.cuda_stream)
+    a = torch.randint(0, 256, (10_007,), dtype=torch.uint8).pin_memory()
+    b = torch.zeros_like(a).pin_memory()
+    d1, d2 = torch.zeros(10_007, dtype=torch.uint8, device=DEV), torch.zeros(10_007, dtype=torch.uint8, device=DEV)
+    torch.cuda.synchronize()
+    for dst, src in ((d1, a), (d2, d1), (b, d2)):
+        assert L.lib.tcu_copy_async(dst.data_ptr(), src.data_ptr(), src.numel(), sp) == 0
+    st.synchronize()
+    assert torch.equal(a, b)
+    assert L.lib.tcu_copy_async(d1.data_ptr() + 1, a.data_ptr() + 3, 5, sp) == 0
+    st.synchronize()
+    assert torch.equal(d1[1:6].cpu(), a[3:8]) and torch.equal(d1[6:].cpu(), a[6:]) and int(d1[0]) == int(a[0])
+
+
+def test_a_dropped_server_leaves_no_work_behind():
+    """A server that goes away with batches in flight has waited for every slot."""
+    from tcuscan_b200 import serve
+
+    x = torch.randint(-8, 9, (1 << 24,), dtype=torch.int8, device=DEV)
+    m = torch.ones(1 << 22, dtype=torch.int8, device=DEV)
+    for _ in range(3):
+        srv = serve.Server(DEV, budget_bytes=1 << 30, slots=3)
+        for _ in range(4):
+            srv.submit("scan", x)
+            srv.submit("compress", x[:1 << 22], m)
+        srv.step()
+        streams = [sl.stream for sl in srv.slots]
+        assert srv.inflight
+        del srv
+        assert all(s.query() for s in streams)
