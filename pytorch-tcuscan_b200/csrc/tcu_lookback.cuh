@@ -200,8 +200,8 @@ __device__ __forceinline__ V wg_lookback(int64_t tid, V agg_inc, V start, TileDe
 // it are still to come (fp16 flag segmented scan of 2^26 elements 139 -> 132 us;
 // uneven fp32 rows and sorted bounds without a difference).  Full scans, whose
 // stops are inclusive prefixes with every tile behind them published, keep the
-// form above: 2^20 fp16 10.45 us against 10.52 with this one, and 10.30 since
-// it looks for no segment starts.
+// form above: 2^20 fp16 10.45 us against 10.52 with this one, and since it looks
+// for no segment starts 10.31 (10.39 with that look, both sides in turn).
 template <typename V>
 __device__ __forceinline__ V wg_lookback_nearest(int64_t tid, V agg_inc, V start, TileDesc* descs, uint32_t epoch,
                                                  const WaitCtx& wc, LbScratch* sc, int wg_thread, uint32_t bar_id,

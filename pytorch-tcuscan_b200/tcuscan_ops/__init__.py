@@ -661,8 +661,8 @@ def _bounds_input(indptr, device, where):
 # SIMT kernels (tcu_seg_sum_rows / tcu_spmv_rows: per-tile start/end bitmaps)
 # instead of the tensor-core segmented sum; 0 = every length, a negative
 # value = none (the tensor-core path for every length).  Measured on
-# B200 at 2^28 fp16 (geometric segment lengths): the bitmap path takes 0.71 /
-# 0.25 / 0.20 ms at mean 4 / 64 / 1024, the tensor-core path 0.48 / 0.36 ms
+# B200 at 2^28 fp16 (geometric segment lengths): the bitmap path takes 0.60 /
+# 0.22 / 0.19 ms at mean 4 / 64 / 1024, the tensor-core path 0.48 / 0.36 ms
 # at mean 64 / 1024, so the split path serves every length by default.
 ROWS_MAX_MEAN = int(os.environ.get("TCU_ROWS_MAX_MEAN", "0"))
 
